@@ -39,6 +39,7 @@ JIT_HEADERS = {
     "common.cuh": os.path.join(CSRC, "common.cuh"),
     "kernels.cuh": os.path.join(CSRC, "kernels.cuh"),
     "trace_common.cuh": os.path.join(CSRC, "trace_common.cuh"),
+    "quotient.cuh": os.path.join(CSRC, "quotient.cuh"),
     "ray_fp64.cuh": os.path.join(CSRC, "ray_fp64.cuh"),
     "mixed.cuh": os.path.join(CSRC, "mixed.cuh"),
     "mixed32.cuh": os.path.join(CSRC, "mixed32.cuh"),
