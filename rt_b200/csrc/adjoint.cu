@@ -590,7 +590,7 @@ int rtb_adjoint_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb
     c->fixes = fixes;
     c->beams_in.assign(beams, beams + n_beams);
     if ((st = check_beams(beams, n_beams, n_rays, c->beams_h)) != RTB_OK ||
-        (st = prepare_scheme(c->surf.data(), n_surfaces, fixes, 0, c->ps)) != RTB_OK) {
+        (st = prepare_scheme(c->surf.data(), n_surfaces, fixes, 0, RTB_FP64, c->ps)) != RTB_OK) {
         delete c;
         return st;
     }
@@ -697,7 +697,7 @@ int rtb_adjoint_forward(rtb_adjoint* c, const double* theta, const rtb_rays* ray
             set_param(sf[c->params[j].surface], c->params[j], theta[j]);
         }
     PreparedScheme ps;
-    int st = prepare_scheme(sf.data(), sf.size(), c->fixes, 0, ps);
+    int st = prepare_scheme(sf.data(), sf.size(), c->fixes, 0, RTB_FP64, ps);
     if (st != RTB_OK) return st;
     // a parameter must not switch a surface's algorithm (check_param at create)
     for (size_t k = 0; k < sf.size(); ++k)

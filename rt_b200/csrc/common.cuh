@@ -77,21 +77,28 @@ struct DevSurface {
 
 // A prepared scheme in device memory; the fused kernels copy it to shared
 // memory, the per-surface kernel reads its one surface from global memory.
+// The surfaces come last: only the first scheme_bytes(n_surfaces) bytes are
+// uploaded, copied and given shared memory (C1's seven surfaces 4 KB of 18).
 struct DevScheme {
     int32_t n_surfaces;
     int32_t n_knots;        // doubles per array in the knot buffer
     uint32_t fixes;
     int32_t renorm_lost;
     int32_t pad[4];
-    DevSurface s[RTB_MAX_SURFACES];
     // FP32-state engine: the first non-Aux surface's transform in FP64 (from
     // the entrance frame), from which each beam's offset is made, and the
     // transform of the Aux surfaces after the last non-Aux one (tail_on).
     double m0[9], off0[3];
     double tail_m[9], tail_off[3];
     int32_t tail_on, pad_tail[3];
+    DevSurface s[RTB_MAX_SURFACES];
 };
 static_assert(sizeof(DevScheme) % 16 == 0, "DevScheme is copied to shared memory in 16-byte words");
+constexpr unsigned kSchemeHeader = sizeof(DevScheme) - RTB_MAX_SURFACES * sizeof(DevSurface);
+static_assert(kSchemeHeader % 16 == 0, "the surfaces follow the header without a gap");
+__host__ __device__ constexpr unsigned scheme_bytes(int n_surfaces) {
+    return (kSchemeHeader + (unsigned)n_surfaces * (unsigned)sizeof(DevSurface) + 15u) / 16u * 16u;
+}
 
 // Beam table on the device (first ray and orders of each beam).
 struct DevBeam {

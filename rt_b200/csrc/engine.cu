@@ -204,15 +204,12 @@ void asphere_sag_bounds(DevSurface& s) {
 }
 
 void mixed_constants(DevSurface& s) {
-    asphere_sag_bounds(s);
     s.inv_c = (s.c != 0.0) ? 1.0 / s.c : 0.0;
     s.inv_gr = (s.gr_const != 0.0) ? 1.0 / s.gr_const : 0.0;
     s.f_c = (float)s.c;
     s.f_k1 = (float)s.k1;
     s.f_cR = (float)s.cR;
     s.f_inv_c = (float)s.inv_c;
-    s.f_sag_lo = (float)s.sag_lo;
-    s.f_sag_hi = (float)s.sag_hi;
     s.f_size0 = (float)s.size[0];
     s.f_pad = 0.0f;
     for (int i = 0; i < RTB_MAX_POLY; ++i) {
@@ -237,7 +234,7 @@ static bool surface_finite(const rtb_surface& in) {
     return in.type != RTB_GRATING || std::isfinite(in.gr_const);
 }
 
-int prepare_surface(const rtb_surface& in, DevSurface& s, KnotBuf& knots) {
+int prepare_surface(const rtb_surface& in, int precision, DevSurface& s, KnotBuf& knots) {
     if (in.type != RTB_AUX_TYPE && !surface_finite(in)) return RTB_BAD_VALUE;
     bool non_aux = in.type != RTB_AUX_TYPE;
     int st = surface_from_params(non_aux ? in.cls : RTB_AUX_CLASS, in.params, s);
@@ -262,6 +259,10 @@ int prepare_surface(const rtb_surface& in, DevSurface& s, KnotBuf& knots) {
         s.center[i] = in.center[i];
     }
     mixed_constants(s);
+    // thousands of square roots per asphere, which only the mixed engines read
+    if (precision != RTB_FP64) asphere_sag_bounds(s);
+    s.f_sag_lo = (float)s.sag_lo;
+    s.f_sag_hi = (float)s.sag_hi;
     s.n1_off = s.n2_off = 0;
     s.n1_n = s.n2_n = 1;
     if (in.type == RTB_LENS || in.type == RTB_GRATING) {
@@ -351,8 +352,8 @@ void beam_frame(const DevScheme& sch, const double center[3], DevBeam& d) {
     }
 }
 
-int prepare_scheme_into(const rtb_surface* surf, size_t n, uint32_t fixes, int renorm_lost, DevScheme& sch,
-                        KnotBuf& knots) {
+int prepare_scheme_into(const rtb_surface* surf, size_t n, uint32_t fixes, int renorm_lost, int precision,
+                        DevScheme& sch, KnotBuf& knots) {
     if (!surf || n == 0 || n > RTB_MAX_SURFACES) return RTB_BAD_VALUE;
     std::memset(&sch, 0, sizeof(sch));
     const double unit[3] = {0.0, 1.0, 0.0};  // offset 0: a harmless single value for unused tables
@@ -360,7 +361,7 @@ int prepare_scheme_into(const rtb_surface* surf, size_t n, uint32_t fixes, int r
     int ng = 0, nonaux = 0;
     for (size_t k = 0; k < n; ++k) {
         DevSurface& s = sch.s[k];
-        int st = prepare_surface(surf[k], s, knots);
+        int st = prepare_surface(surf[k], precision, s, knots);
         if (st != RTB_OK) return st;
         s.grating_index = (s.type == RTB_GRATING) ? ng++ : -1;
         if (s.non_aux) ++nonaux;
@@ -421,10 +422,11 @@ int prepare_scheme_into(const rtb_surface* surf, size_t n, uint32_t fixes, int r
     return RTB_OK;
 }
 
-int prepare_scheme(const rtb_surface* surf, size_t n, uint32_t fixes, int renorm_lost, PreparedScheme& out) {
+int prepare_scheme(const rtb_surface* surf, size_t n, uint32_t fixes, int renorm_lost, int precision,
+                   PreparedScheme& out) {
     out.knots.clear();
     KnotBuf kb(out.knots);
-    return prepare_scheme_into(surf, n, fixes, renorm_lost, out.sch, kb);
+    return prepare_scheme_into(surf, n, fixes, renorm_lost, precision, out.sch, kb);
 }
 
 // Natural cubic spline second derivatives: the sequential algorithm of

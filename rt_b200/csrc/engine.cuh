@@ -1,6 +1,7 @@
 // engine.cuh -- host-side state and helpers of the C ABI.
 #pragma once
 
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -52,19 +53,21 @@ struct KnotBuf {
     const double* data() const { return vec ? vec->data() : fixed; }
 };
 
-int prepare_surface(const rtb_surface& in, DevSurface& out, KnotBuf& knots);
+int prepare_surface(const rtb_surface& in, int precision, DevSurface& out, KnotBuf& knots);
 // Every launch of a scheme reads what this prepares: the surfaces' constants,
 // the packed tables (identical tables sharing one copy, the inverse spacing
 // of tables on a uniform grid) and the counts that follow from the sequence.
-int prepare_scheme_into(const rtb_surface* s, size_t n, uint32_t fixes, int renorm_lost, DevScheme& sch,
-                        KnotBuf& knots);
-int prepare_scheme(const rtb_surface* s, size_t n, uint32_t fixes, int renorm_lost, PreparedScheme& out);
+// precision: RTB_FP64 leaves out what only the mixed engines read.
+int prepare_scheme_into(const rtb_surface* s, size_t n, uint32_t fixes, int renorm_lost, int precision,
+                        DevScheme& sch, KnotBuf& knots);
+int prepare_scheme(const rtb_surface* s, size_t n, uint32_t fixes, int renorm_lost, int precision,
+                   PreparedScheme& out);
 int surface_from_params(int cls, const double* params, DevSurface& s);
 int add_table(const rtb_table* t, KnotBuf& knots, int32_t& off, int32_t& cnt);
 int add_table(const rtb_table* t, std::vector<double>& knots, int32_t& off, int32_t& cnt);
 // Sag range of an even asphere over its circular aperture (DevSurface::sag_*).
 void asphere_sag_bounds(DevSurface& s);
-// The mixed engine's per-surface constants: the sag range and inv_c, inv_gr.
+// The mixed engine's per-surface constants: inv_c, inv_gr and the FP32 copies.
 void mixed_constants(DevSurface& s);
 void transform_constants(const double angles_rad[3], const double dist[3], DevSurface& s);
 double scheme_angle_rad(double deg);
@@ -134,7 +137,10 @@ struct Range {
     Range& operator=(const Range&) = delete;
 };
 
-// Everything a trace launch reads, in one pool allocation.
+// Everything a trace launch reads, in one pool allocation: the scheme, its
+// tables and the beam table (one upload), then the counters, the error word
+// and the tile counter (one memset before, one copy back after a launch: a
+// small trace is as long as its stream operations).
 struct TraceArgs {
     DevBuf buf;
     DevScheme* sch;
@@ -143,28 +149,38 @@ struct TraceArgs {
     unsigned long long* counts;
     unsigned* err;
     unsigned long long* tiles;  // tile counter of the fused kernels
-    size_t counts_len;
+    size_t counts_len;          // counters; the error word is the word after them
+    static constexpr size_t kTail = 256;  // bytes after the counters: error word, tile counter 128 bytes on
     int init(const PreparedScheme& ps, const std::vector<DevBeam>& beams_h, cudaStream_t st) {
         size_t n_beams = beams_h.size();
         counts_len = n_beams * (size_t)(3 * ps.sch.n_surfaces + 1);
-        size_t off_knots = (sizeof(DevScheme) + 255) / 256 * 256;
+        size_t off_knots = (scheme_bytes(ps.sch.n_surfaces) + 255) / 256 * 256;
         size_t off_beams = off_knots + (ps.knots.size() * sizeof(double) + 255) / 256 * 256;
         size_t off_counts = off_beams + (n_beams * sizeof(DevBeam) + 255) / 256 * 256;
-        size_t off_err = off_counts + (counts_len * 8 + 255) / 256 * 256;
-        int s = buf.alloc(off_err + 256, st);
+        int s = buf.alloc(off_counts + counts_len * 8 + kTail, st);
         if (s != RTB_OK) return s;
         char* p = buf.as<char>();
         sch = reinterpret_cast<DevScheme*>(p);
         knots = reinterpret_cast<double*>(p + off_knots);
         beams = reinterpret_cast<DevBeam*>(p + off_beams);
         counts = reinterpret_cast<unsigned long long*>(p + off_counts);
-        err = reinterpret_cast<unsigned*>(p + off_err);
-        tiles = reinterpret_cast<unsigned long long*>(p + off_err + 64);
-        RTB_CUDA_TRY(cudaMemcpyAsync(sch, &ps.sch, sizeof(DevScheme), cudaMemcpyHostToDevice, st));
-        RTB_CUDA_TRY(cudaMemcpyAsync(knots, ps.knots.data(), ps.knots.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-        RTB_CUDA_TRY(cudaMemcpyAsync(beams, beams_h.data(), n_beams * sizeof(DevBeam), cudaMemcpyHostToDevice, st));
-        RTB_CUDA_TRY(cudaMemsetAsync(counts, 0, counts_len * 8, st));
-        RTB_CUDA_TRY(cudaMemsetAsync(err, 0, 256, st));  // err and the tile counter
+        err = reinterpret_cast<unsigned*>(counts + counts_len);
+        tiles = counts + counts_len + 16;
+        std::vector<char> h(off_beams + n_beams * sizeof(DevBeam));
+        std::memcpy(h.data(), &ps.sch, scheme_bytes(ps.sch.n_surfaces));
+        std::memcpy(h.data() + off_knots, ps.knots.data(), ps.knots.size() * sizeof(double));
+        std::memcpy(h.data() + off_beams, beams_h.data(), n_beams * sizeof(DevBeam));
+        RTB_CUDA_TRY(cudaMemcpyAsync(p, h.data(), h.size(), cudaMemcpyHostToDevice, st));
+        return clear(st);
+    }
+    // Zero the counters, the error word and the tile counter.
+    int clear(cudaStream_t st) {
+        RTB_CUDA_TRY(cudaMemsetAsync(counts, 0, counts_len * 8 + kTail, st));
+        return RTB_OK;
+    }
+    // The counters and, after them, the error word (counts_len + 1 words).
+    int fetch(unsigned long long* host, cudaStream_t st) const {
+        RTB_CUDA_TRY(cudaMemcpyAsync(host, counts, (counts_len + 1) * 8, cudaMemcpyDeviceToHost, st));
         return RTB_OK;
     }
 };
@@ -195,6 +211,9 @@ int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_
 // `order` (device, n).
 int coherent_order(const GenBeam* d_beams, int n_beams, uint64_t n, const DevRays& rays, uint32_t* order,
                    int chunk_shift, cudaStream_t st);
+// The launch configuration of a trace that names none.
+constexpr int kDefaultBlock = 256;
+int default_rpt(int precision, uint64_t n_rays);
 // Status and statistics from the per-(beam, stage) counts.
 int trace_result(const PreparedScheme& ps, const unsigned long long* counts, unsigned err, int n_beams,
                  rtb_trace_stats* stats);

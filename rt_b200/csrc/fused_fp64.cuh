@@ -44,6 +44,8 @@ __device__ __forceinline__ void f64_surface(const DevSurface& s, int k, uint32_t
 // The surfaces in order, the whole block stepping through them together (a
 // barrier after each; every thread calls run, also without a live ray).
 struct RtSurfacesF64 {
+    static constexpr bool kBaked = false;
+    __device__ __forceinline__ static int renorm_after(const DevScheme* sch, int k) { return sch->s[k].renorm_after; }
     __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots, const DevBeam* beams,
                                                int b, double lam, unsigned* err, f64::Ray& r, int& stage) {
         for (int k = 0; k < sch->n_surfaces; ++k) {
@@ -69,9 +71,8 @@ __device__ __forceinline__ void fused_fp64(const DevScheme* __restrict__ g_sch, 
                                            unsigned long long* counts, unsigned* err, int state_out,
                                            FrameArgs frame, TileSched ts) {
     const double* s_knots;
-    const DevScheme* sch = stage_scheme(g_sch, knots, s_knots);
-    const int ns = sch->n_surfaces;
-    const int n_stages = 3 * ns;
+    const DevScheme* sch = stage_scheme<Surfaces::kBaked>(g_sch, knots, ts, s_knots);
+    const int n_stages = 3 * ts.n_surfaces;
     const uint64_t block_rays = (uint64_t)blockDim.x * (uint64_t)ts.rpt;
     const uint64_t n_tiles = (in.n + block_rays - 1) / block_rays;
     __shared__ unsigned long long s_tile;
@@ -106,7 +107,7 @@ __device__ __forceinline__ void fused_fp64(const DevScheme* __restrict__ g_sch, 
             if (have) {
                 if (stage >= 0) {
                     ev = true;
-                    if (sch->renorm_lost) f64::renormalize(r, sch->s[stage / 3].renorm_after);
+                    if (sch->renorm_lost) f64::renormalize(r, Surfaces::renorm_after(sch, stage / 3));
                     out.flag[oi] = 0;
                     out.lost_stage[oi] = (uint8_t)stage;
                     key = b * (n_stages + 1) + stage;

@@ -201,10 +201,12 @@ std::string scheme_source(const DevScheme& sch, int precision) {
     const bool bake = bake_values();
     const std::string S = bake ? "k_surfaces()[" : "sch->s[";
     const std::string F = bake ? "k_fixes" : "sch->fixes";
+    const std::string kBaked = bake ? "    static constexpr bool kBaked = true;\n"
+                                    : "    static constexpr bool kBaked = false;\n";
     if (precision == RTB_MIXED) {
         src = "#include \"mixed.cuh\"\n" + (bake ? surface_constants(sch) : std::string()) +
               "namespace rtb {\n"
-              "struct SchemeSurfaces {\n"
+              "struct SchemeSurfaces {\n" + kBaked +
               "    __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots,\n"
               "        const BeamCtx& bc, double lam, mx::TableMemo& memo, mx::Ray& r, int& stage) {\n";
         for (int k = 0; k < sch.n_surfaces; ++k) {
@@ -219,7 +221,7 @@ std::string scheme_source(const DevScheme& sch, int precision) {
     } else if (precision == RTB_MIXED32) {
         src = "#include \"mixed32.cuh\"\n" + (bake ? surface_constants(sch) : std::string()) +
               "namespace rtb {\n"
-              "struct SchemeSurfaces32 {\n"
+              "struct SchemeSurfaces32 {\n" + kBaked +
               "    __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots,\n"
               "        const BeamCtx& bc, const double* off0, double lam, mx::TableMemo& memo, m32::Ray& r,\n"
               "        mx::Ray& q, int& stage) {\n";
@@ -236,7 +238,9 @@ std::string scheme_source(const DevScheme& sch, int precision) {
     } else {
         src = "#include \"fused_fp64.cuh\"\n" + (bake ? surface_constants(sch) : std::string()) +
               "namespace rtb {\n"
-              "struct SchemeSurfacesF64 {\n"
+              "struct SchemeSurfacesF64 {\n" + kBaked +
+              "    __device__ __forceinline__ static int renorm_after(const DevScheme* sch, int k) {\n"
+              "        return " + S + "k].renorm_after;\n    }\n"
               "    __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots,\n"
               "        const DevBeam* beams, int b, double lam, unsigned* err, f64::Ray& r, int& stage) {\n";
         for (int k = 0; k < sch.n_surfaces; ++k) {
@@ -483,7 +487,7 @@ int rtb_specialize(const rtb_surface* surfaces, size_t n_surfaces, uint32_t fixe
     if (note && note_len > 0) note[0] = 0;
     if (precision != RTB_FP64 && precision != RTB_MIXED && precision != RTB_MIXED32) return RTB_BAD_VALUE;
     PreparedScheme ps;
-    int st = prepare_scheme(surfaces, n_surfaces, fixes, 0, ps);
+    int st = prepare_scheme(surfaces, n_surfaces, fixes, 0, precision, ps);
     if (st != RTB_OK) return st;
     std::string why;
     st = compile_scheme(ps.sch, precision, &why);
@@ -495,7 +499,7 @@ int rtb_adjoint_specialize(const rtb_surface* surfaces, size_t n_surfaces, uint3
                            size_t note_len) {
     if (note && note_len > 0) note[0] = 0;
     PreparedScheme ps;
-    int st = prepare_scheme(surfaces, n_surfaces, fixes, 0, ps);
+    int st = prepare_scheme(surfaces, n_surfaces, fixes, 0, RTB_FP64, ps);
     if (st != RTB_OK) return st;
     std::string why;
     st = compile_adjoint(ps.sch, &why);

@@ -26,10 +26,13 @@ struct FrameArgs {
 };
 
 #ifndef __CUDACC_RTC__
-// Size of the dynamic shared memory the fused kernels use.
-inline size_t fused_smem_bytes(int n_knots) {
-    return ((sizeof(DevScheme) + 15) / 16) * 16 + sizeof(double) * (size_t)n_knots;
+// Size of the dynamic shared memory the fused kernels use, and the size that
+// decides whether a scheme's tables fit a block: that of a full scheme,
+// whatever its number of surfaces.
+inline size_t fused_smem_bytes(int n_surfaces, int n_knots) {
+    return scheme_bytes(n_surfaces) + sizeof(double) * (size_t)n_knots;
 }
+inline size_t fused_smem_limit(int n_knots) { return fused_smem_bytes(RTB_MAX_SURFACES, n_knots); }
 #endif
 
 // Scheduling of the persistent fused kernels: `next` is a counter of tiles
@@ -42,6 +45,8 @@ inline size_t fused_smem_bytes(int n_knots) {
 // `rows` (mixed kernels, may be NULL): the rays in tracing order as row
 // blocks (Row64 for RTB_MIXED, Row32 for RTB_MIXED32, rowpipe.cuh), read in
 // place of `in`.  out_by_slot: outputs go to the tracing slot instead.
+// n_surfaces, n_knots: the scheme's, as launch arguments so that its staging
+// does not wait for a first read of the scheme.
 struct TileSched {
     unsigned long long* next;
     int rpt;
@@ -49,8 +54,8 @@ struct TileSched {
     int in_by_slot;
     const void* rows;
     int out_by_slot;
+    int n_surfaces, n_knots;
 };
-constexpr int kDefaultRpt = 2;
 
 // One surface of a throughput curve (k_qe_curves): its QE table in the knot
 // array, and for a grating the order and rule parameters, angles in radians.

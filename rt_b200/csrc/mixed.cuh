@@ -572,6 +572,7 @@ __device__ __forceinline__ int mx_surface(const DevSurface& s, int k, uint32_t f
 // scheme (jit.cpp) passes a policy whose run() calls mx_surface with each
 // surface's FixedShape in turn.
 struct RtSurfaces {
+    static constexpr bool kBaked = false;
     __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots, const BeamCtx& bc,
                                                double lam, mx::TableMemo& memo, mx::Ray& r, int& stage) {
         for (int k = 0; k < sch->n_surfaces && stage == -1; ++k)
@@ -596,9 +597,9 @@ __device__ __forceinline__ void fused_mixed(const DevScheme* __restrict__ g_sch,
                                             unsigned long long* counts, unsigned* err, int state_out,
                                             FrameArgs frame, TileSched ts) {
     const double* s_knots;
-    const DevScheme* sch = stage_scheme(g_sch, knots, s_knots);
-    const int n_stages = 3 * sch->n_surfaces;
-    RowLoop rows(ts, in.n, warp_row_buffer<Row64>(sch->n_knots), (unsigned)sizeof(Row64), err);
+    const DevScheme* sch = stage_scheme<Surfaces::kBaked>(g_sch, knots, ts, s_knots);
+    const int n_stages = 3 * ts.n_surfaces;
+    RowLoop rows(ts, in.n, warp_row_buffer<Row64>(ts.n_surfaces, ts.n_knots), (unsigned)sizeof(Row64), err);
     const int lane = threadIdx.x & 31;
     BeamCursor cur;
     while (rows.begin()) {

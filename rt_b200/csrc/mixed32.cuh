@@ -229,6 +229,7 @@ __device__ __forceinline__ int m32_surface(const DevSurface& s, int k, uint32_t 
 // surface's structure read from the scheme; jit.cpp writes the same with a
 // FixedShape per surface).
 struct Rt32Surfaces {
+    static constexpr bool kBaked = false;
     __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots, const BeamCtx& bc,
                                                const double* off0, double lam, mx::TableMemo& memo, m32::Ray& r,
                                                mx::Ray& q, int& stage) {
@@ -247,9 +248,9 @@ __device__ __forceinline__ void fused_mixed32(const DevScheme* __restrict__ g_sc
                                               unsigned long long* counts, unsigned* err, int state_out,
                                               FrameArgs frame, TileSched ts) {
     const double* s_knots;
-    const DevScheme* sch = stage_scheme(g_sch, knots, s_knots);
-    const int n_stages = 3 * sch->n_surfaces;
-    RowLoop rows(ts, in.n, warp_row_buffer<Row32>(sch->n_knots), (unsigned)sizeof(Row32), err);
+    const DevScheme* sch = stage_scheme<Surfaces::kBaked>(g_sch, knots, ts, s_knots);
+    const int n_stages = 3 * ts.n_surfaces;
+    RowLoop rows(ts, in.n, warp_row_buffer<Row32>(ts.n_surfaces, ts.n_knots), (unsigned)sizeof(Row32), err);
     const int lane = threadIdx.x & 31;
     BeamCursor cur;
     while (rows.begin()) {

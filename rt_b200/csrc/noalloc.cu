@@ -88,7 +88,7 @@ extern "C" RTB_API int rtb_trace_out_noalloc(const rtb_surface* surfaces, size_t
     // the launch configuration rtb_trace_out accepts (launch_trace)
     const int threads = (opts->block_size > 0) ? opts->block_size : 256;
     if (threads != 128 && threads != 256 && !(mixed && threads == 512)) return RTB_BAD_VALUE;
-    const int rpt = (opts->rays_per_thread > 0) ? opts->rays_per_thread : kDefaultRpt;
+    const int rpt = (opts->rays_per_thread > 0) ? opts->rays_per_thread : default_rpt(opts->precision, in->n);
     if (rpt < 1 || rpt > 64) return RTB_BAD_VALUE;
     const size_t ns1 = 3 * n_surfaces + 1;
     if (layout(0, n_beams, n_beams * ns1).total > RTB_NOALLOC_SCRATCH_BYTES) return RTB_BAD_VALUE;
@@ -106,14 +106,14 @@ extern "C" RTB_API int rtb_trace_out_noalloc(const rtb_surface* surfaces, size_t
     // (prepare_scheme_into), its tables packed at their final offset
     const size_t knots_at = layout(0, 0, 0).knots;
     KnotBuf kb(reinterpret_cast<double*>(h_stage + knots_at), RTB_NOALLOC_MAX_KNOTS);
-    if ((st = prepare_scheme_into(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, h_scheme, kb)) !=
+    if ((st = prepare_scheme_into(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, opts->precision, h_scheme, kb)) !=
         RTB_OK)
         return st;
     const size_t n_knots = kb.size();
     const Layout l = layout(n_knots, n_beams, n_beams * ns1);
     if (l.total > RTB_NOALLOC_SCRATCH_BYTES) return RTB_BAD_VALUE;
-    const size_t smem = fused_smem_bytes((int)n_knots);
-    if (smem > (size_t)engine().max_smem_optin) return RTB_BAD_VALUE;
+    if (fused_smem_limit((int)n_knots) > (size_t)engine().max_smem_optin) return RTB_BAD_VALUE;
+    const size_t smem = fused_smem_bytes((int)n_surfaces, (int)n_knots);
     std::memcpy(h_stage, &h_scheme, sizeof(DevScheme));
     DevBeam* beams_h = reinterpret_cast<DevBeam*>(h_stage + l.beams);
     uint64_t prev_end = 0;
@@ -165,7 +165,7 @@ extern "C" RTB_API int rtb_trace_out_noalloc(const rtb_surface* surfaces, size_t
     kern<<<grid_for(in->n, threads * rpt, per_sm), threads, smem, s>>>(
         reinterpret_cast<const DevScheme*>(d), reinterpret_cast<const double*>(d + l.knots),
         reinterpret_cast<const DevBeam*>(d + l.beams), (int)n_beams, ri, ro, counts_d, err_d,
-        opts->state_out ? 1 : 0, frame, TileSched{tiles_d, rpt, nullptr, 0});
+        opts->state_out ? 1 : 0, frame, TileSched{tiles_d, rpt, nullptr, 0, nullptr, 0, (int)n_surfaces, (int)n_knots});
     RTB_CUDA_TRY(cudaGetLastError());
     unsigned long long* counts_h = reinterpret_cast<unsigned long long*>(h_stage + l.counts);
     unsigned err = 0;

@@ -44,7 +44,7 @@ struct rtb_plan {
     cudaGraphExec_t exec = nullptr;
     bool graph_stale = true;
     bool ran = false;
-    int32_t block = 256, rpt = kDefaultRpt;
+    int32_t block = kDefaultBlock, rpt = 1;
     uint64_t key = 0;
     std::string jit_note;            // why the generic kernel is launched ("" if specialised)
 };
@@ -108,21 +108,19 @@ size_t rays_bytes(uint64_t n, bool full) {
 
 // The stream operations of one run.
 int enqueue_run(rtb_plan* p, const FrameArgs& frame, cudaStream_t s) {
-    RTB_CUDA_TRY(cudaMemsetAsync(p->args.counts, 0, p->args.counts_len * 8, s));
-    RTB_CUDA_TRY(cudaMemsetAsync(p->args.err, 0, 256, s));  // error word and tile counter
+    int st = p->args.clear(s);
+    if (st != RTB_OK) return st;
     rtb_trace_opts o = p->opts;
     o.block_size = p->block;
     o.rays_per_thread = p->rpt;
     const bool by_slot = p->opts.out_order == RTB_OUT_SLOT;
-    int st = p->rows    ? launch_trace(p->ps, p->args, (int)p->n_beams, o, p->in, p->out, frame, s, p->order, true,
+    st = p->rows        ? launch_trace(p->ps, p->args, (int)p->n_beams, o, p->in, p->out, frame, s, p->order, true,
                                        p->rows, by_slot)
              : p->order ? launch_trace(p->ps, p->args, (int)p->n_beams, o, p->in_slot, p->out, frame, s, p->order,
                                        true, nullptr, by_slot)
                         : launch_trace(p->ps, p->args, (int)p->n_beams, o, p->in, p->out, frame, s);
     if (st != RTB_OK) return st;
-    RTB_CUDA_TRY(cudaMemcpyAsync(p->h_counts, p->args.counts, p->args.counts_len * 8, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaMemcpyAsync(p->h_counts + p->args.counts_len, p->args.err, 4, cudaMemcpyDeviceToHost, s));
-    return RTB_OK;
+    return p->args.fetch(p->h_counts, s);
 }
 
 int capture(rtb_plan* p) {
@@ -205,7 +203,7 @@ int rtb_plan_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
     // lock (NVRTC takes up to a second or so; other calls need not wait)
     if (specialize_enabled()) {
         PreparedScheme pre;
-        if (prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, pre) == RTB_OK)
+        if (prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, opts->precision, pre) == RTB_OK)
             compile_scheme(pre.sch, opts->precision, nullptr);
     }
     Lock l;
@@ -231,7 +229,7 @@ int rtb_plan_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
     p->n_rays = beams[n_beams - 1].first_ray + beams[n_beams - 1].n_rays;
     std::vector<GenBeam> gb;
     uint64_t total = 0;
-    if ((st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, p->ps)) != RTB_OK ||
+    if ((st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, opts->precision, p->ps)) != RTB_OK ||
         (st = check_beams(beams, n_beams, p->n_rays, p->beams_h, &p->ps.sch)) != RTB_OK ||
         (st = gen_beams(beams, n_beams, p->n_rays, gb, &total)) != RTB_OK) {
         delete p;
@@ -243,9 +241,10 @@ int rtb_plan_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
         delete p;
         return st;
     }
+    p->rpt = default_rpt(opts->precision, p->n_rays);
     if (opts->block_size > 0 || opts->rays_per_thread > 0) {
-        p->block = opts->block_size > 0 ? opts->block_size : 256;
-        p->rpt = opts->rays_per_thread > 0 ? opts->rays_per_thread : kDefaultRpt;
+        if (opts->block_size > 0) p->block = opts->block_size;
+        if (opts->rays_per_thread > 0) p->rpt = opts->rays_per_thread;
         if (!config_ok(*p, p->block, p->rpt)) {
             delete p;
             return RTB_BAD_VALUE;

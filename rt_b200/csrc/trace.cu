@@ -109,6 +109,19 @@ int gen_beams(const rtb_beam* beams, size_t n_beams, size_t n_rays, std::vector<
     return RTB_OK;
 }
 
+// Rows of 32 rays that a warp (mixed) or rays that a thread (FP64) takes at a
+// time.  More of them amortise the tile counter, whose one address serves all
+// warps; fewer spread a small trace over the chip.  On C1 in a plan, ms at 1 /
+// 2 / 4 rows: mixed 2e5 rays (1.3 rows per resident warp) 0.051 / 0.054 /
+// 0.071, 6e5 (4) 0.076 / 0.075 / 0.087, 2e6 (13) 0.182 / 0.148 / 0.138, 1e8
+// 5.73 / 3.87 / 3.87; FP64, whose blocks share a tile and step through the
+// surfaces together, 2e5 0.075 / 0.079 / 0.102, 2e7 2.88 / 2.89 / 2.92.
+int default_rpt(int precision, uint64_t n_rays) {
+    if (precision == RTB_FP64) return 1;
+    const uint64_t warps = (uint64_t)engine().sm_count * 32, rows = n_rays / 32;
+    return rows < 2 * warps ? 1 : rows < 8 * warps ? 2 : 4;
+}
+
 int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_trace_opts& o, const DevRays& in,
                  const DevRays& out, const FrameArgs& frame, cudaStream_t st, const uint32_t* order,
                  bool in_by_slot, const void* rows, bool out_by_slot) {
@@ -126,14 +139,16 @@ int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_
         const bool mixed = o.precision == RTB_MIXED || m32;
         if (!mixed && o.precision != RTB_FP64) return RTB_BAD_VALUE;
         if (rows && !mixed) return RTB_BAD_VALUE;
-        const int threads = (o.block_size > 0) ? o.block_size : 256;
+        const int threads = (o.block_size > 0) ? o.block_size : kDefaultBlock;
         if (threads != 128 && threads != 256 && !(mixed && threads == 512)) return RTB_BAD_VALUE;
-        const int rpt = (o.rays_per_thread > 0) ? o.rays_per_thread : kDefaultRpt;
+        const int rpt = (o.rays_per_thread > 0) ? o.rays_per_thread : default_rpt(o.precision, in.n);
         if (rpt < 1 || rpt > 64) return RTB_BAD_VALUE;
-        size_t smem = fused_smem_bytes(ps.sch.n_knots);
-        if (rows) smem = (smem + 127) / 128 * 128 + (m32 ? row_buffers_bytes<Row32>(threads)
-                                                         : row_buffers_bytes<Row64>(threads));
-        if (smem > (size_t)engine().max_smem_optin) return RTB_BAD_VALUE;
+        auto with_rows = [&](size_t b) {
+            if (!rows) return b;
+            return (b + 127) / 128 * 128 + (m32 ? row_buffers_bytes<Row32>(threads) : row_buffers_bytes<Row64>(threads));
+        };
+        if (with_rows(fused_smem_limit(ps.sch.n_knots)) > (size_t)engine().max_smem_optin) return RTB_BAD_VALUE;
+        const size_t smem = with_rows(fused_smem_bytes(ps.sch.n_surfaces, ps.sch.n_knots));
         const void* kern = ps.scheme_kernel ? ps.scheme_kernel
                            : m32           ? reinterpret_cast<const void*>(k_fused_mixed32)
                            : mixed         ? reinterpret_cast<const void*>(k_fused_mixed)
@@ -153,7 +168,8 @@ int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_
         unsigned* err = a.err;
         int state_out = o.state_out ? 1 : 0;
         FrameArgs fr = frame;
-        TileSched ts{a.tiles, rpt, order, in_by_slot ? 1 : 0, rows, out_by_slot ? 1 : 0};
+        TileSched ts{a.tiles, rpt, order, in_by_slot ? 1 : 0, rows, out_by_slot ? 1 : 0, ps.sch.n_surfaces,
+                     ps.sch.n_knots};
         void* params[] = {&sch, &knots, &beams, &nb, &rin, &rout, &counts, &err, &state_out, &fr, &ts};
         RTB_CUDA_TRY(cudaLaunchKernel(kern, dim3(grid), dim3(threads), params, smem, st));
     } else {
@@ -197,6 +213,31 @@ int trace_result(const PreparedScheme& ps, const unsigned long long* counts, uns
     return RTB_OK;
 }
 
+// A one-shot trace of device rays: `out` may be `in`.
+static int trace_device(const rtb_surface* surfaces, size_t n_surfaces, const rtb_beam* beams, size_t n_beams,
+                        const rtb_trace_opts* opts, const rtb_rays* in, const rtb_rays* out, rtb_trace_stats* stats,
+                        void* stream) {
+    Lock l;
+    int st = ensure_init();
+    if (st != RTB_OK) return st;
+    cudaStream_t s = stream ? (cudaStream_t)stream : engine().stream;
+    PreparedScheme ps;
+    if ((st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, opts->precision, ps)) !=
+            RTB_OK ||
+        (st = attach_compiled(ps, *opts)) != RTB_OK)
+        return st;
+    std::vector<DevBeam> db;
+    if ((st = check_beams(beams, n_beams, in->n, db, &ps.sch)) != RTB_OK) return st;
+    TraceArgs a;
+    if ((st = a.init(ps, db, s)) != RTB_OK) return st;
+    FrameArgs frame = frame_args(opts);
+    if ((st = launch_trace(ps, a, (int)n_beams, *opts, dev_rays(in), dev_rays(out), frame, s)) != RTB_OK) return st;
+    std::vector<unsigned long long> counts(a.counts_len + 1);
+    if ((st = a.fetch(counts.data(), s)) != RTB_OK) return st;
+    RTB_CUDA_TRY(cudaStreamSynchronize(s));
+    return trace_result(ps, counts.data(), (unsigned)counts[a.counts_len], (int)n_beams, stats);
+}
+
 }  // namespace rtb
 
 using namespace rtb;
@@ -225,27 +266,7 @@ int rtb_trace(const rtb_surface* surfaces, size_t n_surfaces, const rtb_beam* be
               const rtb_trace_opts* opts, const rtb_rays* rays, rtb_trace_stats* stats, void* stream) {
     Range range("rtb_trace");
     if (!opts || !rays || !rays->flag || !rays->lost_stage) return RTB_BAD_VALUE;
-    Lock l;
-    int st = ensure_init();
-    if (st != RTB_OK) return st;
-    cudaStream_t s = stream ? (cudaStream_t)stream : engine().stream;
-    PreparedScheme ps;
-    if ((st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, ps)) != RTB_OK ||
-        (st = attach_compiled(ps, *opts)) != RTB_OK)
-        return st;
-    std::vector<DevBeam> db;
-    if ((st = check_beams(beams, n_beams, rays->n, db, &ps.sch)) != RTB_OK) return st;
-    TraceArgs a;
-    if ((st = a.init(ps, db, s)) != RTB_OK) return st;
-    FrameArgs frame = frame_args(opts);
-    DevRays dr = dev_rays(rays);
-    if ((st = launch_trace(ps, a, (int)n_beams, *opts, dr, dr, frame, s)) != RTB_OK) return st;
-    std::vector<unsigned long long> counts(a.counts_len);
-    unsigned err = 0;
-    RTB_CUDA_TRY(cudaMemcpyAsync(counts.data(), a.counts, a.counts_len * 8, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaMemcpyAsync(&err, a.err, 4, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaStreamSynchronize(s));
-    return trace_result(ps, counts.data(), err, (int)n_beams, stats);
+    return trace_device(surfaces, n_surfaces, beams, n_beams, opts, rays, rays, stats, stream);
 }
 
 int rtb_trace_out(const rtb_surface* surfaces, size_t n_surfaces, const rtb_beam* beams, size_t n_beams,
@@ -253,26 +274,7 @@ int rtb_trace_out(const rtb_surface* surfaces, size_t n_surfaces, const rtb_beam
                   void* stream) {
     Range range("rtb_trace_out");
     if (!opts || !in || !out || !in->flag || !out->flag || !out->lost_stage || in->n != out->n) return RTB_BAD_VALUE;
-    Lock l;
-    int st = ensure_init();
-    if (st != RTB_OK) return st;
-    cudaStream_t s = stream ? (cudaStream_t)stream : engine().stream;
-    PreparedScheme ps;
-    if ((st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, ps)) != RTB_OK ||
-        (st = attach_compiled(ps, *opts)) != RTB_OK)
-        return st;
-    std::vector<DevBeam> db;
-    if ((st = check_beams(beams, n_beams, in->n, db, &ps.sch)) != RTB_OK) return st;
-    TraceArgs a;
-    if ((st = a.init(ps, db, s)) != RTB_OK) return st;
-    FrameArgs frame = frame_args(opts);
-    if ((st = launch_trace(ps, a, (int)n_beams, *opts, dev_rays(in), dev_rays(out), frame, s)) != RTB_OK) return st;
-    std::vector<unsigned long long> counts(a.counts_len);
-    unsigned err = 0;
-    RTB_CUDA_TRY(cudaMemcpyAsync(counts.data(), a.counts, a.counts_len * 8, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaMemcpyAsync(&err, a.err, 4, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaStreamSynchronize(s));
-    return trace_result(ps, counts.data(), err, (int)n_beams, stats);
+    return trace_device(surfaces, n_surfaces, beams, n_beams, opts, in, out, stats, stream);
 }
 
 int rtb_ccd_frame(const rtb_rays* rays, const rtb_ccd* ccd, uint32_t* counts, uint64_t* n_outside, void* stream) {
@@ -350,7 +352,7 @@ namespace rtb {
 int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_beam* beams, size_t n_beams,
                     const rtb_trace_opts* opts, const rtb_rays* h, rtb_trace_stats* stats, size_t chunk) {
     PreparedScheme ps;
-    int st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, ps);
+    int st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, opts->precision, ps);
     if (st == RTB_OK) st = attach_compiled(ps, *opts);
     if (st != RTB_OK) return st;
     std::vector<DevBeam> db;
@@ -427,7 +429,7 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
         const size_t nb = sl.beam_ids.size();
         for (size_t b = 0; b < nb; ++b)
             for (int k = 0; k < ns1; ++k) total[(size_t)sl.beam_ids[b] * ns1 + k] += sl.h_counts[b * ns1 + k];
-        err_all |= (unsigned)(sl.h_counts[nb * ns1] & 0xffffffffu);
+        err_all |= (unsigned)(sl.h_counts[sl.args.counts_len] & 0xffffffffu);
         if (sl.h_flag) std::memcpy(h->flag + sl.start, sl.h_flag, sl.cnt);
         if (sl.h_lost) std::memcpy(h->lost_stage + sl.start, sl.h_lost, sl.cnt);
         sl.beam_ids.clear();
@@ -478,9 +480,7 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
         } else
             RTB_CUDA_TRY(cudaMemsetAsync(sl.r.lost_stage, RTB_NOT_LOST, cnt, s));
         RTB_CUDA_TRY(cudaMemcpyAsync(sl.args.beams, sl.h_beams, nb * sizeof(DevBeam), cudaMemcpyHostToDevice, s));
-        sl.args.counts_len = nb * ns1;
-        RTB_CUDA_TRY(cudaMemsetAsync(sl.args.counts, 0, sl.args.counts_len * 8, s));
-        RTB_CUDA_TRY(cudaMemsetAsync(sl.args.err, 0, 256, s));  // error word and tile counter
+        if ((st = sl.args.clear(s)) != RTB_OK) break;
         if ((st = launch_trace(ps, sl.args, (int)nb, o, sl.r, sl.r, frame, s)) != RTB_OK) break;
         int nout = o.state_out ? 6 : 2;
         for (int j = 0; j < nout; ++j)
@@ -489,8 +489,7 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
         if (h->lost_stage)
             RTB_CUDA_TRY(cudaMemcpyAsync(sl.h_lost ? sl.h_lost : h->lost_stage + start, sl.r.lost_stage, cnt,
                                          cudaMemcpyDeviceToHost, s));
-        RTB_CUDA_TRY(cudaMemcpyAsync(sl.h_counts, sl.args.counts, sl.args.counts_len * 8, cudaMemcpyDeviceToHost, s));
-        RTB_CUDA_TRY(cudaMemcpyAsync(sl.h_counts + sl.args.counts_len, sl.args.err, 4, cudaMemcpyDeviceToHost, s));
+        if ((st = sl.args.fetch(sl.h_counts, s)) != RTB_OK) break;
         start += cnt;
         ++it;
     }

@@ -127,16 +127,18 @@ __device__ __forceinline__ void frame_add(bool good, double X, double Y, const F
 }
 
 // Copy the scheme and the knot tables into shared memory (fused kernels).
+// A kernel with the surfaces baked in copies only the header.
+template <bool kBaked>
 __device__ __forceinline__ const DevScheme* stage_scheme(const DevScheme* sch, const double* knots,
-                                                         const double*& s_knots) {
+                                                         const TileSched& ts, const double*& s_knots) {
     extern __shared__ __align__(16) unsigned char smem[];
     DevScheme* s_sch = reinterpret_cast<DevScheme*>(smem);
-    double* kn = reinterpret_cast<double*>(smem + ((sizeof(DevScheme) + 15) / 16) * 16);
+    double* kn = reinterpret_cast<double*>(smem + scheme_bytes(ts.n_surfaces));
     const int4* src = reinterpret_cast<const int4*>(sch);
     int4* dst = reinterpret_cast<int4*>(smem);
-    for (int j = threadIdx.x; j < (int)(sizeof(DevScheme) / 16); j += blockDim.x) dst[j] = src[j];
-    int nk = sch->n_knots;
-    for (int j = threadIdx.x; j < nk; j += blockDim.x) kn[j] = knots[j];
+    const int words = (int)((kBaked ? kSchemeHeader : scheme_bytes(ts.n_surfaces)) / 16);
+    for (int j = threadIdx.x; j < words; j += blockDim.x) dst[j] = src[j];
+    for (int j = threadIdx.x; j < ts.n_knots; j += blockDim.x) kn[j] = knots[j];
     __syncthreads();
     s_knots = kn;
     return s_sch;
