@@ -9,7 +9,9 @@
 //
 // reference_order() replays the Rearrange calls of a whole trace from the
 // per-ray lost stages (one partition per stage with losses, all beams at
-// once), giving the order in which the reference's Beam::Save writes rays.
+// once, in one cooperative launch), giving the order in which the reference's
+// Beam::Save writes rays.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include "engine.cuh"
@@ -32,15 +34,6 @@ __device__ __forceinline__ int seg_of(const Seg* segs, int n_segs, uint64_t k) {
         if (segs[mid].start <= k) lo = mid; else hi = mid - 1;
     }
     return lo;
-}
-
-__global__ void k_mark_stage(uint64_t n, const Seg* segs, int n_segs, const uint32_t* order, const uint8_t* lost_stage,
-                             int stage, uint32_t* mark) {
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)blockDim.x * gridDim.x) {
-        int s = seg_of(segs, n_segs, k);
-        bool in = k < segs[s].start + segs[s].ng;
-        mark[k] = (in && lost_stage[segs[s].start + order[k]] == stage) ? 1u : 0u;
-    }
 }
 
 // Per segment: lost count = rank[start+ng] - rank[start].
@@ -85,16 +78,6 @@ __device__ __forceinline__ void pair_front(uint64_t k, const Seg* segs, int n_se
     swap(k, slot_pos[start + r]);
 }
 
-__global__ void k_swap_order(uint64_t n, const Seg* segs, int n_segs, const uint32_t* mark, const uint32_t* rank,
-                             const uint64_t* seg_lost, const uint64_t* slot_pos, uint32_t* order) {
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)blockDim.x * gridDim.x)
-        pair_front(k, segs, n_segs, mark, rank, seg_lost, slot_pos, [&](uint64_t a, uint64_t b) {
-            uint32_t t = order[a];
-            order[a] = order[b];
-            order[b] = t;
-        });
-}
-
 struct Arr7 {
     double* a[7];
 };
@@ -111,18 +94,6 @@ __global__ void k_swap_arrays(uint64_t n, const Seg* segs, const uint32_t* mark,
             flag[a] = 1;
             flag[b] = 0;
         });
-}
-
-__global__ void k_seg_update(Seg* segs, int n_segs, const uint64_t* seg_lost) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < n_segs) segs[s].ng -= seg_lost[s];
-}
-
-__global__ void k_iota(uint64_t n, const Seg* segs, int n_segs, uint32_t* order) {
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)blockDim.x * gridDim.x) {
-        int s = seg_of(segs, n_segs, k);
-        order[k] = (uint32_t)(k - segs[s].start);
-    }
 }
 
 __global__ void k_mark_flags(uint64_t ng, const char* flag, uint32_t* mark) {
@@ -162,33 +133,257 @@ struct Work {
 
 }  // namespace
 
+namespace {
+
+// The replay of a whole trace's Rearrange calls (k_replay).  A segment (beam)
+// is cut into tiles of kTile positions; `stage` holds the lost stage of the
+// ray at each position, a tile's kTile bytes together, and follows the swaps.
+constexpr int kTile = 4096, kReplayThreads = 256, kPer = kTile / kReplayThreads;
+
+struct ReplaySeg {
+    uint64_t start;          // position of its first ray
+    uint32_t n, ng;          // rays, good ones before the stage at hand
+    uint32_t lost, pairs;    // of the stage at hand: rays lost, swaps
+    uint32_t tile0, pad;     // its first tile
+};
+
+struct Replay {
+    ReplaySeg* segs;
+    int n_segs, n_stages;
+    uint32_t n_tiles;
+    uint64_t n;
+    const uint8_t* lost_stage;
+    uint32_t* order;         // beam-local index of the ray at each position
+    uint8_t* stage;
+    uint32_t* tile_lost;     // rays of a tile lost at the stage at hand
+    uint32_t *front, *back;  // the k-th lost ray's position, and its partner's (at segment start + k)
+    unsigned* any;           // bit mask of the stages that lost rays
+};
+
+__device__ __forceinline__ int seg_of_tile(const Replay& r, uint32_t t) {
+    int lo = 0, hi = r.n_segs - 1;
+    while (lo < hi) {  // the last segment that starts at or before tile t: empty ones have no tiles
+        const int mid = (lo + hi + 1) >> 1;
+        if (r.segs[mid].tile0 <= t) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Bit i: of the thread's kPer positions from j0 on, position j0 + i lies
+// before `end` and its ray was lost at stage `st`.
+__device__ __forceinline__ unsigned lost_bits(const Replay& r, uint32_t t, uint32_t j0, uint32_t end, unsigned st) {
+    if (j0 >= end) return 0;
+    const uint4 w = *reinterpret_cast<const uint4*>(r.stage + (size_t)t * kTile + threadIdx.x * kPer);
+    const unsigned v[4] = {w.x, w.y, w.z, w.w};
+    unsigned bits = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const unsigned eq = __vcmpeq4(v[q], st * 0x01010101u) & 0x08040201u;
+        bits |= ((eq | eq >> 8 | eq >> 16 | eq >> 24) & 0xfu) << (4 * q);
+    }
+    const uint32_t left = end - j0;
+    return left < kPer ? bits & ((1u << left) - 1u) : bits;
+}
+
+// Sum over the block, to every thread.
+__device__ __forceinline__ unsigned block_sum(unsigned v, unsigned* s_warp) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    unsigned sum = 0;
+    for (int w = 0; w < kReplayThreads / 32; ++w) sum += s_warp[w];
+    __syncthreads();
+    return sum;
+}
+
+// Every stage in turn, the whole grid together; a stage that lost no ray is
+// passed over.  Per stage: count each tile's lost rays; with the sums before
+// its tiles (and so the number of rays that stay, N'), every block lists the
+// front's lost rays by rank and the back's good rays by rank from the back;
+// swap the pairs, spread over all of the segment's tiles.  Bound by latency:
+// three grid barriers a stage and the scattered reads of the swaps.  C1's 31
+// beams, 4e6 rays, losses at 5 of 21 stages: 0.18 ms; 1.5 ms as six kernels
+// and a library scan over 32-bit marks for each of the 21 stages, mostly the
+// gaps between 168 launches.
+__global__ void __launch_bounds__(kReplayThreads, 4) k_replay(Replay r) {
+    auto grid = cooperative_groups::this_grid();
+    __shared__ unsigned s_warp[kReplayThreads / 32];
+    using Scan = cub::BlockScan<unsigned, kReplayThreads>;
+    __shared__ typename Scan::TempStorage s_scan;
+    // a contiguous run of tiles per block: the sums before them are made once
+    // per segment and block
+    const uint32_t t0 = (uint32_t)((uint64_t)r.n_tiles * blockIdx.x / gridDim.x);
+    const uint32_t t1 = (uint32_t)((uint64_t)r.n_tiles * (blockIdx.x + 1) / gridDim.x);
+    const int first_seg = t0 < t1 ? seg_of_tile(r, t0) : 0;
+    // the segment of the next tile; tiles are visited in order
+    auto advance = [&](int s, uint32_t t) {
+        while (s + 1 < r.n_segs && r.segs[s + 1].tile0 <= t) ++s;
+        return s;
+    };
+    // positions outside every segment, relative to the segment before them
+    for (int g = (int)blockIdx.x - 1; g < r.n_segs; g += (int)gridDim.x) {
+        const uint64_t from = g < 0 ? 0 : r.segs[g].start + r.segs[g].n, base = r.segs[g < 0 ? 0 : g].start;
+        const uint64_t to = g + 1 < r.n_segs ? r.segs[g + 1].start : r.n;
+        for (uint64_t k = from + threadIdx.x; k < to; k += kReplayThreads) r.order[k] = (uint32_t)(k - base);
+    }
+    unsigned seen[3] = {0, 0, 0};
+    int s = first_seg;
+    for (uint32_t t = t0; t < t1; ++t) {
+        s = advance(s, t);
+        const uint32_t j0 = (t - r.segs[s].tile0) * kTile, len = min((uint32_t)kTile, r.segs[s].n - j0);
+        const uint64_t at = r.segs[s].start + j0;
+        uint8_t v[kPer];  // all loads in flight at once
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const uint32_t j = threadIdx.x + i * kReplayThreads;
+            v[i] = j < len ? r.lost_stage[at + j] : (uint8_t)RTB_NOT_LOST;
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const uint32_t j = threadIdx.x + i * kReplayThreads;
+            if (j >= len) break;
+            r.stage[(size_t)t * kTile + j] = v[i];
+            r.order[at + j] = j0 + j;
+            if (v[i] < r.n_stages) {
+                const unsigned bit = 1u << (v[i] & 31);
+                if (v[i] < 32) seen[0] |= bit;
+                else if (v[i] < 64) seen[1] |= bit;
+                else seen[2] |= bit;
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const unsigned m = __reduce_or_sync(0xffffffffu, seen[q]);
+        if (m && (threadIdx.x & 31) == 0) atomicOr(r.any + q, m);
+    }
+    grid.sync();
+    for (int st = 0; st < r.n_stages; ++st) {
+        if (!(r.any[st >> 5] >> (st & 31) & 1u)) continue;
+        s = first_seg;
+        for (uint32_t t = t0; t < t1; ++t) {
+            s = advance(s, t);
+            const uint32_t j0 = (t - r.segs[s].tile0) * kTile + threadIdx.x * kPer;
+            const unsigned c = block_sum(__popc(lost_bits(r, t, j0, r.segs[s].ng, st)), s_warp);
+            if (threadIdx.x == 0) r.tile_lost[t] = c;
+        }
+        grid.sync();
+        s = first_seg;
+        int sums_of = -1;
+        uint32_t before = 0, total = 0;
+        for (uint32_t t = t0; t < t1; ++t) {
+            s = advance(s, t);
+            const ReplaySeg& g = r.segs[s];
+            if (sums_of != s) {
+                const uint32_t g1 = g.tile0 + (uint32_t)(((uint64_t)g.n + kTile - 1) / kTile);
+                unsigned b = 0, a = 0;
+                for (uint32_t q = g.tile0 + threadIdx.x; q < g1; q += kReplayThreads) {
+                    const unsigned c = r.tile_lost[q];
+                    a += c;
+                    if (q < t) b += c;
+                }
+                before = block_sum(b, s_warp);
+                total = block_sum(a, s_warp);
+                sums_of = s;
+            }
+            if (t == g.tile0 && threadIdx.x == 0) r.segs[s].lost = total;
+            const uint32_t in_tile = r.tile_lost[t], ng = g.ng, keep = ng - total;  // keep: N'
+            const uint32_t tile_j = (t - g.tile0) * kTile;
+            const bool holds_keep = total && tile_j <= keep && keep - tile_j < kTile;
+            // a front tile without lost rays and a back tile without good ones list nothing
+            const bool idle =
+                total == 0 || tile_j >= ng ||
+                (!holds_keep && (tile_j < keep ? in_tile == 0 : in_tile == min((uint32_t)kTile, ng - tile_j)));
+            if (!idle) {
+                const uint32_t j0 = tile_j + threadIdx.x * kPer;
+                const unsigned bits = lost_bits(r, t, j0, ng, st);
+                unsigned rank;
+                Scan(s_scan).ExclusiveSum(__popc(bits), rank);
+                __syncthreads();
+                rank += before;  // rays of the segment lost before position j0
+                uint32_t* const front = r.front + g.start;
+                uint32_t* const back = r.back + g.start;
+                const unsigned have = j0 >= ng ? 0u : ng - j0 < kPer ? (1u << (ng - j0)) - 1u : (1u << kPer) - 1u;
+                // the positions before N'
+                const unsigned fore = j0 >= keep ? 0u : keep - j0 < kPer ? (1u << (keep - j0)) - 1u : (1u << kPer) - 1u;
+                for (unsigned m = bits & fore; m; m &= m - 1)
+                    front[rank + __popc(bits & ((m & -m) - 1u))] = j0 + __ffs(m) - 1;
+                for (unsigned m = have & ~bits & ~fore; m; m &= m - 1) {
+                    const uint32_t j = j0 + __ffs(m) - 1;
+                    back[(ng - 1 - j) - (total - rank - __popc(bits & ((m & -m) - 1u)))] = j;
+                }
+                if (j0 <= keep && keep - j0 < kPer) r.segs[s].pairs = rank + __popc(bits & fore);
+            } else if (total == 0 && t == g.tile0 && threadIdx.x == 0) {
+                r.segs[s].pairs = 0;
+            }
+            before += in_tile;
+        }
+        grid.sync();
+        s = first_seg;
+        for (uint32_t t = t0; t < t1; ++t) {
+            s = advance(s, t);
+            ReplaySeg& g = r.segs[s];
+            // the pairs spread over all of the segment's tiles
+            const uint32_t pairs = g.pairs, tiles = (uint32_t)(((uint64_t)g.n + kTile - 1) / kTile);
+            for (uint64_t k = (uint64_t)(t - g.tile0) * kReplayThreads + threadIdx.x; k < pairs;
+                 k += (uint64_t)tiles * kReplayThreads) {
+                const uint32_t a = r.front[g.start + k], b = r.back[g.start + k];
+                const uint32_t o = r.order[g.start + a];
+                r.order[g.start + a] = r.order[g.start + b];
+                r.order[g.start + b] = o;
+                // position b leaves the good rays: its stage is not read again
+                r.stage[(size_t)g.tile0 * kTile + a] = r.stage[(size_t)g.tile0 * kTile + b];
+            }
+            if (t == g.tile0 && threadIdx.x == 0) g.ng -= g.lost;
+        }
+        grid.sync();
+    }
+}
+
+}  // namespace
+
 int reference_order(const DevBeam* h_beams, int n_beams, int n_stages, const DevRays& rays, uint32_t* order,
                     cudaStream_t st) {
-    uint64_t n = rays.n;
+    const uint64_t n = rays.n;
     if (n == 0) return RTB_OK;
     if (n > 0xFFFFFFFFull) return RTB_BAD_VALUE;
-    std::vector<Seg> segs(n_beams);
+    std::vector<ReplaySeg> segs(n_beams);
+    uint64_t tiles = 0;
     for (int b = 0; b < n_beams; ++b) {
-        segs[b].start = h_beams[b].first_ray;
-        segs[b].ng = h_beams[b].n_rays;
-        if (b > 0 && segs[b].start < segs[b - 1].start + segs[b - 1].ng) return RTB_BAD_VALUE;
+        const uint32_t nr = (uint32_t)h_beams[b].n_rays;
+        segs[b] = ReplaySeg{h_beams[b].first_ray, nr, nr, 0, 0, (uint32_t)tiles, 0};
+        if (b > 0 && segs[b].start < segs[b - 1].start + segs[b - 1].n) return RTB_BAD_VALUE;
+        tiles += (nr + (uint64_t)kTile - 1) / kTile;
     }
-    Work w;
-    int s = w.init(n, n_beams, st);
+    auto al = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t o_any = 0, o_segs = 256, o_lost = o_segs + al(n_beams * sizeof(ReplaySeg)),
+                 o_stage = o_lost + al(tiles * 4), o_front = o_stage + al(tiles * kTile), o_back = o_front + al(n * 4);
+    DevBuf buf;
+    int s = buf.alloc(o_back + al(n * 4), st);
     if (s != RTB_OK) return s;
-    RTB_CUDA_TRY(cudaMemcpyAsync(w.segs, segs.data(), n_beams * sizeof(Seg), cudaMemcpyHostToDevice, st));
-    unsigned grid = grid_for(n, 256, 8);
-    unsigned sg = (unsigned)((n_beams + 255) / 256);
-    k_iota<<<grid, 256, 0, st>>>(n, w.segs, n_beams, order);
-    for (int stage = 0; stage < n_stages; ++stage) {
-        k_mark_stage<<<grid, 256, 0, st>>>(n, w.segs, n_beams, order, rays.lost_stage, stage, w.mark);
-        if ((s = w.exclusive_scan(n, st)) != RTB_OK) return s;
-        k_seg_counts<<<sg, 256, 0, st>>>(w.segs, n_beams, w.rank, w.mark, w.seg_lost);
-        k_back_slots<<<grid, 256, 0, st>>>(n, w.segs, n_beams, w.mark, w.rank, w.seg_lost, w.slot);
-        k_swap_order<<<grid, 256, 0, st>>>(n, w.segs, n_beams, w.mark, w.rank, w.seg_lost, w.slot, order);
-        k_seg_update<<<sg, 256, 0, st>>>(w.segs, n_beams, w.seg_lost);
-    }
-    RTB_CUDA_TRY(cudaGetLastError());
+    char* p = buf.as<char>();
+    Replay r;
+    r.segs = reinterpret_cast<ReplaySeg*>(p + o_segs);
+    r.n_segs = n_beams;
+    r.n_stages = n_stages;
+    r.n_tiles = (uint32_t)tiles;
+    r.n = n;
+    r.lost_stage = rays.lost_stage;
+    r.order = order;
+    r.stage = reinterpret_cast<uint8_t*>(p + o_stage);
+    r.tile_lost = reinterpret_cast<uint32_t*>(p + o_lost);
+    r.front = reinterpret_cast<uint32_t*>(p + o_front);
+    r.back = reinterpret_cast<uint32_t*>(p + o_back);
+    r.any = reinterpret_cast<unsigned*>(p + o_any);
+    RTB_CUDA_TRY(cudaMemsetAsync(r.any, 0, 256, st));
+    RTB_CUDA_TRY(cudaMemcpyAsync(r.segs, segs.data(), n_beams * sizeof(ReplaySeg), cudaMemcpyHostToDevice, st));
+    int per_sm = 0;
+    RTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_replay, kReplayThreads, 0));
+    // no more blocks than tiles: the barriers cost by the block
+    unsigned blocks = grid_for(n, kTile, per_sm < 4 ? per_sm : 4);
+    void* args[] = {&r};
+    RTB_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_replay), dim3(blocks),
+                                             dim3(kReplayThreads), args, 0, st));
     return RTB_OK;
 }
 
