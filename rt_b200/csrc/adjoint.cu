@@ -46,7 +46,7 @@ constexpr int kMeritThreads = 256;
 constexpr int kMeritParts = 32;    // fixed split of each group's rays (deterministic sums)
 
 // The forward through any scheme (adjoint_rev.cuh).
-__global__ void __launch_bounds__(256) k_adj_forward(AdjArgs a, DevRays in, unsigned long long* counts,
+__global__ void __launch_bounds__(kAdjForwardThreads, 4) k_adj_forward(AdjArgs a, DevRays in, unsigned long long* counts,
                                                      unsigned* err) {
     adj_forward<RtAdjForward>(a, in, counts, err);
 }
@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_backward(AdjArgs a, cons
         if (!__any_sync(0xffffffffu, act)) continue;
         const double lam = act ? a.lambda[i] : 0.0;
         const int b = act ? beam_of(a.beams, a.n_beams, i) : 0;
+        const unsigned live = __ballot_sync(0xffffffffu, act);
         for (int k = ns - 1; k >= 0; --k) {
             const DevSurface& s = sch->s[k];
             double st[6];
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_backward(AdjArgs a, cons
                 ad::RayD<kAdjW> r;
                 if (act) {
                     ad::load_state(st, sd, r, t1, t2);
-                    ad::surface_step(s, table[e], sch->fixes, a.knots, adj_order(s, a.beams, b), lam, r);
+                    ad::surface_step(s, table[e], sch->fixes, a.knots, adj_order(s, a.beams, b), lam, live, r);
                 }
                 // the last surface's output is the CCD-plane point: only X, Y
                 // carry adjoints.  Components are picked with selects (run-time
@@ -219,7 +220,7 @@ __global__ void k_adj_sum_partials(const double* partial, int n_blocks, int P, d
 // Forward-mode sensitivities along one parameter direction, through the whole
 // scheme from checkpoint 0 (the input rays); table[k]: surface k's constants
 // along that direction.
-__global__ void __launch_bounds__(kAdjThreads) k_adj_jvp(AdjArgs a, const ad::SurfD<1>* table, double* dX,
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_jvp(AdjArgs a, const ad::SurfD<1>* table, double* dX,
                                                          double* dY) {
     adj_jvp<RtAdjJvp>(a, table, dX, dY);
 }
@@ -717,9 +718,10 @@ int rtb_adjoint_forward(rtb_adjoint* c, const double* theta, const rtb_rays* ray
         unsigned long long* counts = c->d_counts;
         unsigned* err = c->d_err;
         void* args[] = {&a, &in, &counts, &err};
-        RTB_CUDA_TRY(cudaLaunchKernel(c->fwd_kernel, dim3(adj_grid(c->n, 256)), dim3(256), args, 0, s));
+        RTB_CUDA_TRY(cudaLaunchKernel(c->fwd_kernel, dim3(adj_grid(c->n, kAdjForwardThreads)),
+                                      dim3(kAdjForwardThreads), args, 0, s));
     } else {
-        k_adj_forward<<<adj_grid(c->n, 256), 256, 0, s>>>(a, in, c->d_counts, c->d_err);
+        k_adj_forward<<<adj_grid(c->n, kAdjForwardThreads), kAdjForwardThreads, 0, s>>>(a, in, c->d_counts, c->d_err);
     }
     RTB_CUDA_TRY(cudaGetLastError());
     if (X) RTB_CUDA_TRY(cudaMemcpyAsync(X, c->d_X, c->n * 8, cudaMemcpyDeviceToDevice, s));

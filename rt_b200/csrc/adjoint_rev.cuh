@@ -26,6 +26,12 @@ namespace rtb {
 
 constexpr int kAdjThreads = 128;
 constexpr int kAdjWarps = kAdjThreads / 32;
+// The forward runs at 64 registers, 32 warps an SM, as the fused FP64 kernel
+// does (C4, 2e6 rays: 0.36 ms, 0.38 at the 110 registers the compiler takes
+// unbounded); the reverse sweep at 128 and 16 warps (0.70; 0.90 at three
+// blocks an SM, 0.75 at five, where it spills); the sensitivities unbounded at
+// two blocks (0.88; 0.94 at the 128 registers of four).
+constexpr int kAdjForwardThreads = 256;
 
 struct AdjArgs {
     const DevScheme* sch;
@@ -75,10 +81,18 @@ struct AdjShape {
 // Surface k (structure Sh) of the forward on one ray: its input state
 // stored as checkpoint k, then the plain FP64 engine's surface.  -1 while
 // the ray survives, the stage that lost it, or -2 (a wavelength outside a
-// table).
+// table).  live: the lanes that call it; on return, those of them that
+// survive.  They meet again after the intersection, whose root iterations
+// they leave at different steps, and before the last normalisation: without
+// that each group of lanes ran the rest of the scheme by itself (C4: the
+// detector's plane took the instructions of three surfaces at 9 lanes of 32),
+// 0.39 ms against 0.36 for 2e6 rays.  The fused FP64 kernel, whose blocks meet
+// after every surface, and the reverse sweep, whose warps do, lose by it
+// (2.87 -> 2.96 and 0.70 -> 0.75 ms): there the groups hide each other's
+// latency within the surface.
 template <class Sh>
 __device__ __forceinline__ int fwd_surface(const AdjArgs& a, int k, size_t i, int b, double lam, unsigned* err,
-                                           f64::Ray& r) {
+                                           unsigned& live, f64::Ray& r) {
     double* c = a.ckpt + (size_t)k * 6 * a.n + i;
     c[0] = r.X;
     c[a.n] = r.Y;
@@ -91,24 +105,34 @@ __device__ __forceinline__ int fwd_surface(const AdjArgs& a, int k, size_t i, in
     f64::transform<Sh>(s, r);
     f64::normalize(r.cX, r.cY, r.cZ);
     if (!Sh::non_aux(s)) return -1;
-    if (!f64::intersect<Sh>(s, sch->fixes, r)) return 3 * k;
-    if (!f64::aperture_pass(Sh::type(s) == RTB_SHADE, Sh::shape(s), s.size, s.center, r.X, r.Y)) return 3 * k + 1;
-    const int act = f64::action<Sh>(s, a.knots, adj_order(s, a.beams, b), lam, r);
-    if (act == f64::ACT_RANGE) {
-        atomicOr(err, DEV_ERR_OUT_OF_RANGE);
-        return -2;
+    const bool hit = f64::intersect<Sh>(s, sch->fixes, r);
+    __syncwarp(live);
+    int stage = -1;
+    if (!hit) {
+        stage = 3 * k;
+    } else if (!f64::aperture_pass(Sh::type(s) == RTB_SHADE, Sh::shape(s), s.size, s.center, r.X, r.Y)) {
+        stage = 3 * k + 1;
+    } else {
+        const int act = f64::action<Sh>(s, a.knots, adj_order(s, a.beams, b), lam, r);
+        if (act == f64::ACT_RANGE) {
+            atomicOr(err, DEV_ERR_OUT_OF_RANGE);
+            stage = -2;
+        } else if (act == f64::ACT_LOST) {
+            stage = 3 * k + 2;
+        }
     }
-    if (act == f64::ACT_LOST) return 3 * k + 2;
-    f64::normalize(r.cX, r.cY, r.cZ);
-    return -1;
+    live = __ballot_sync(live, stage == -1);
+    if (stage == -1) f64::normalize(r.cX, r.cY, r.cZ);
+    return stage;
 }
 
 // The forward through any scheme, its structure read at run time.
 struct RtAdjForward {
     __device__ __forceinline__ static int run(const AdjArgs& a, size_t i, int b, double lam, unsigned* err,
-                                              f64::Ray& r) {
+                                              unsigned live, f64::Ray& r) {
         int stage = -1;
-        for (int k = 0; k < a.sch->n_surfaces && stage == -1; ++k) stage = fwd_surface<RtShape>(a, k, i, b, lam, err, r);
+        for (int k = 0; k < a.sch->n_surfaces && stage == -1; ++k)
+            stage = fwd_surface<RtShape>(a, k, i, b, lam, err, live, r);
         return stage;
     }
 };
@@ -118,19 +142,22 @@ template <class Surfaces>
 __device__ __forceinline__ void adj_forward(const AdjArgs& a, const DevRays& in, unsigned long long* counts,
                                             unsigned* err) {
     const int n_stages = 3 * a.sch->n_surfaces;
-    for (size_t i = gtid(); i < a.n; i += gstride()) {
-        a.lambda[i] = in.lambda[i];
-        if (in.flag[i] != 1) {
-            a.flag[i] = 0;
-            continue;
+    const int lane = threadIdx.x & 31;
+    for (size_t i0 = gtid() - lane; i0 < a.n; i0 += gstride()) {
+        const size_t i = i0 + lane;
+        const bool have = i < a.n && in.flag[i] == 1;
+        const unsigned live = __ballot_sync(0xffffffffu, have);
+        int stage = -2, b = 0;
+        if (i < a.n) a.lambda[i] = in.lambda[i];
+        if (have) {
+            f64::Ray r{in.X[i], in.Y[i], in.Z[i], in.cX[i], in.cY[i], in.cZ[i]};
+            b = beam_of(a.beams, a.n_beams, i);
+            stage = Surfaces::run(a, i, b, in.lambda[i], err, live, r);
+            a.X[i] = r.X;
+            a.Y[i] = r.Y;
         }
-        f64::Ray r{in.X[i], in.Y[i], in.Z[i], in.cX[i], in.cY[i], in.cZ[i]};
-        const double lam = in.lambda[i];
-        const int b = beam_of(a.beams, a.n_beams, i);
-        const int stage = Surfaces::run(a, i, b, lam, err, r);
-        a.flag[i] = (stage == -1) ? 1 : 0;
-        a.X[i] = r.X;
-        a.Y[i] = r.Y;
+        __syncwarp();
+        if (i < a.n) a.flag[i] = (stage == -1) ? 1 : 0;
         // one atomic per distinct counter in the warp (the rays of a beam
         // mostly share theirs)
         count_event(stage != -2, b * (n_stages + 1) + (stage >= 0 ? stage : n_stages), counts);
@@ -141,16 +168,16 @@ __device__ __forceinline__ void adj_forward(const AdjArgs& a, const DevRays& in,
 // table[k] holds the surface's constants along the direction.
 template <class Sh>
 __device__ __forceinline__ void jvp_surface(const AdjArgs& a, int k, const ad::SurfD<1>* table, int b, double lam,
-                                            ad::RayD<1>& r) {
+                                            unsigned live, ad::RayD<1>& r) {
     const DevSurface& s = a.sch->s[k];
-    ad::surface_step<1, Sh>(s, table[k], a.sch->fixes, a.knots, adj_order(s, a.beams, b), lam, r);
+    ad::surface_step<1, Sh>(s, table[k], a.sch->fixes, a.knots, adj_order(s, a.beams, b), lam, live, r);
 }
 
 // The sensitivities through any scheme, its structure read at run time.
 struct RtAdjJvp {
     __device__ __forceinline__ static void run(const AdjArgs& a, const ad::SurfD<1>* table, int b, double lam,
-                                               ad::RayD<1>& r) {
-        for (int k = 0; k < a.sch->n_surfaces; ++k) jvp_surface<RtShape>(a, k, table, b, lam, r);
+                                               unsigned live, ad::RayD<1>& r) {
+        for (int k = 0; k < a.sch->n_surfaces; ++k) jvp_surface<RtShape>(a, k, table, b, lam, live, r);
     }
 };
 
@@ -159,10 +186,13 @@ struct RtAdjJvp {
 // entrance rays (checkpoint 0); 0 for lost rays.
 template <class Surfaces>
 __device__ __forceinline__ void adj_jvp(const AdjArgs& a, const ad::SurfD<1>* table, double* dX, double* dY) {
-    for (size_t i = gtid(); i < a.n; i += gstride()) {
-        if (a.flag[i] != 1) {
-            dX[i] = 0.0;
-            dY[i] = 0.0;
+    const int lane = threadIdx.x & 31;
+    for (size_t i0 = gtid() - lane; i0 < a.n; i0 += gstride()) {
+        const size_t i = i0 + lane;
+        const bool have = i < a.n && a.flag[i] == 1;
+        const unsigned live = __ballot_sync(0xffffffffu, have);
+        if (!have) {
+            if (i < a.n) dX[i] = dY[i] = 0.0;
             continue;
         }
         const double lam = a.lambda[i];
@@ -175,7 +205,7 @@ __device__ __forceinline__ void adj_jvp(const AdjArgs& a, const ad::SurfD<1>* ta
         for (int c = 0; c < 6; ++c) st[c] = a.ckpt[(size_t)c * a.n + i];
         ad::RayD<1> r;
         ad::load_state(st, sd, r);
-        Surfaces::run(a, table, b, lam, r);
+        Surfaces::run(a, table, b, lam, live, r);
         dX[i] = r.X.d[0];
         dY[i] = r.Y.d[0];
     }

@@ -432,11 +432,11 @@ std::string adjoint_source(const DevScheme& sch) {
         "namespace rtb {\n"
         "struct SchemeAdjForward {\n"
         "    __device__ __forceinline__ static int run(const AdjArgs& a, size_t i, int b, double lam, unsigned* err,\n"
-        "                                              f64::Ray& r) {\n"
+        "                                              unsigned live, f64::Ray& r) {\n"
         "        int stage = -1;\n";
     for (int k = 0; k < sch.n_surfaces; ++k)
         src += "        if (stage == -1) stage = fwd_surface<" + adj_shape(sch.s[k]) + ">(a, " + std::to_string(k) +
-               ", i, b, lam, err, r);\n";
+               ", i, b, lam, err, live, r);\n";
     src += "        return stage;\n    }\n};\n"
            "struct SchemeAdjJvp {\n"
            "    __device__ __forceinline__ static void run(const AdjArgs& a, const ad::SurfD<1>* table, int b,\n"
@@ -449,13 +449,13 @@ std::string adjoint_source(const DevScheme& sch) {
     for (int k = sch.n_surfaces - 1; k >= 0; --k)
         src += "        rev_surface<" + adj_shape(sch.s[k]) + ">(a, " + std::to_string(k) + ", ray, lane, acc_row);\n";
     src += std::string("    }\n};\n}  // namespace rtb\n"
-                       "extern \"C\" __global__ void __launch_bounds__(256) ") + kAdjForwardName +
+                       "extern \"C\" __global__ void __launch_bounds__(rtb::kAdjForwardThreads, 4) ") + kAdjForwardName +
            "(rtb::AdjArgs a, rtb::DevRays in,\n        unsigned long long* counts, unsigned* err) {\n"
            "    rtb::adj_forward<rtb::SchemeAdjForward>(a, in, counts, err);\n}\n"
            "extern \"C\" __global__ void __launch_bounds__(rtb::kAdjThreads, 4) " + kAdjReverseName +
            "(rtb::AdjArgs a,\n        const double* gX, const double* gY, double* partial) {\n"
            "    rtb::adj_reverse<rtb::SchemeAdjSurfaces>(a, gX, gY, partial);\n}\n"
-           "extern \"C\" __global__ void __launch_bounds__(rtb::kAdjThreads) " + kAdjJvpName +
+           "extern \"C\" __global__ void __launch_bounds__(rtb::kAdjThreads, 2) " + kAdjJvpName +
            "(rtb::AdjArgs a,\n        const rtb::ad::SurfD<1>* table, double* dX, double* dY) {\n"
            "    rtb::adj_jvp<rtb::SchemeAdjJvp>(a, table, dX, dY);\n}\n";
     return src;
