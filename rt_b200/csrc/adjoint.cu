@@ -137,7 +137,6 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_backward(AdjArgs a, cons
         if (!__any_sync(0xffffffffu, act)) continue;
         const double lam = act ? a.lambda[i] : 0.0;
         const int b = act ? beam_of(a.beams, a.n_beams, i) : 0;
-        const unsigned live = __ballot_sync(0xffffffffu, act);
         for (int k = ns - 1; k >= 0; --k) {
             const DevSurface& s = sch->s[k];
             double st[6];
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_backward(AdjArgs a, cons
                 ad::RayD<kAdjW> r;
                 if (act) {
                     ad::load_state(st, sd, r, t1, t2);
-                    ad::surface_step(s, table[e], sch->fixes, a.knots, adj_order(s, a.beams, b), lam, live, r);
+                    ad::surface_step(s, table[e], sch->fixes, a.knots, adj_order(s, a.beams, b), lam, r);
                 }
                 // the last surface's output is the CCD-plane point: only X, Y
                 // carry adjoints.  Components are picked with selects (run-time

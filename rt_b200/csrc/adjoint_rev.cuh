@@ -168,16 +168,16 @@ __device__ __forceinline__ void adj_forward(const AdjArgs& a, const DevRays& in,
 // table[k] holds the surface's constants along the direction.
 template <class Sh>
 __device__ __forceinline__ void jvp_surface(const AdjArgs& a, int k, const ad::SurfD<1>* table, int b, double lam,
-                                            unsigned live, ad::RayD<1>& r) {
+                                            ad::RayD<1>& r) {
     const DevSurface& s = a.sch->s[k];
-    ad::surface_step<1, Sh>(s, table[k], a.sch->fixes, a.knots, adj_order(s, a.beams, b), lam, live, r);
+    ad::surface_step<1, Sh>(s, table[k], a.sch->fixes, a.knots, adj_order(s, a.beams, b), lam, r);
 }
 
 // The sensitivities through any scheme, its structure read at run time.
 struct RtAdjJvp {
     __device__ __forceinline__ static void run(const AdjArgs& a, const ad::SurfD<1>* table, int b, double lam,
-                                               unsigned live, ad::RayD<1>& r) {
-        for (int k = 0; k < a.sch->n_surfaces; ++k) jvp_surface<RtShape>(a, k, table, b, lam, live, r);
+                                               ad::RayD<1>& r) {
+        for (int k = 0; k < a.sch->n_surfaces; ++k) jvp_surface<RtShape>(a, k, table, b, lam, r);
     }
 };
 
@@ -186,13 +186,10 @@ struct RtAdjJvp {
 // entrance rays (checkpoint 0); 0 for lost rays.
 template <class Surfaces>
 __device__ __forceinline__ void adj_jvp(const AdjArgs& a, const ad::SurfD<1>* table, double* dX, double* dY) {
-    const int lane = threadIdx.x & 31;
-    for (size_t i0 = gtid() - lane; i0 < a.n; i0 += gstride()) {
-        const size_t i = i0 + lane;
-        const bool have = i < a.n && a.flag[i] == 1;
-        const unsigned live = __ballot_sync(0xffffffffu, have);
-        if (!have) {
-            if (i < a.n) dX[i] = dY[i] = 0.0;
+    for (size_t i = gtid(); i < a.n; i += gstride()) {
+        if (a.flag[i] != 1) {
+            dX[i] = 0.0;
+            dY[i] = 0.0;
             continue;
         }
         const double lam = a.lambda[i];
@@ -205,7 +202,7 @@ __device__ __forceinline__ void adj_jvp(const AdjArgs& a, const ad::SurfD<1>* ta
         for (int c = 0; c < 6; ++c) st[c] = a.ckpt[(size_t)c * a.n + i];
         ad::RayD<1> r;
         ad::load_state(st, sd, r);
-        Surfaces::run(a, table, b, lam, live, r);
+        Surfaces::run(a, table, b, lam, r);
         dX[i] = r.X.d[0];
         dY[i] = r.Y.d[0];
     }
