@@ -8,15 +8,14 @@
 // ray's state (X Y Z cX cY cZ) at the input of every surface -- 48 bytes x
 // surfaces per ray.
 //
-// Per ray, surfaces last to first: surface k is recomputed from checkpoint k
-// and the adjoint of its output state is carried back through its stages in
-// reverse order (ray_rev.cuh), giving the adjoint of its input state and of
-// the constants its parameters move, in one sweep.  Rays are taken 32 at a
-// time per warp, every lane of a warp the same number of steps, so the warp
-// sums each parameter's contributions over its lanes with a shuffle tree
-// into its row in shared memory; the block adds its warps' rows in order and
-// writes one partial per parameter, which the caller sums in block order: the
-// gradient is reproducible.
+// Per ray, surfaces last to first: the adjoint of surface k's output state
+// (checkpoint k + 1) is carried back through its stages in reverse order to
+// its input state (checkpoint k; ray_rev.cuh), giving the adjoint of its input state and of
+// the constants its parameters move, in one sweep.  Each thread adds its rays'
+// contributions to a parameter in a shared-memory word of its own, in order;
+// the block adds its threads' words in a fixed order and writes one partial
+// per parameter, which the caller sums in a fixed order: the gradient is
+// reproducible.
 #pragma once
 
 #include "ray_rev.cuh"
@@ -28,8 +27,8 @@ constexpr int kAdjThreads = 128;
 constexpr int kAdjWarps = kAdjThreads / 32;
 // The forward runs at 64 registers, 32 warps an SM, as the fused FP64 kernel
 // does (C4, 2e6 rays: 0.36 ms, 0.38 at the 110 registers the compiler takes
-// unbounded); the reverse sweep at 128 and 16 warps (0.70; 0.90 at three
-// blocks an SM, 0.75 at five, where it spills); the sensitivities unbounded at
+// unbounded); the reverse sweep at 128 and 16 warps (0.47; 0.60 at three
+// blocks an SM, 0.51 at five, where it spills); the sensitivities unbounded at
 // two blocks (0.88; 0.94 at the 128 registers of four).
 constexpr int kAdjForwardThreads = 256;
 
@@ -215,13 +214,18 @@ struct RevRay {
     int b;          // its beam
     double lam;
     rv::RayA adj;   // the adjoint of its state at the output of the next surface to sweep
+    bool have_out;  // that state is known: the last surface's is not kept
+    f64::Ray out;
 };
 
 // Surface k (structure Sh) of the reverse sweep for the warp's rays: the
-// adjoint carried back through it, the contributions to its parameters
-// summed over the warp into the warp's row of shared-memory sums.
+// adjoint carried back through it, the contributions to its parameters added
+// to the thread's sums, acc[j * kAdjThreads] for parameter j.  A load, an add
+// and a store per parameter and ray, where a shuffle tree over the warp took 15
+// instructions: C4, 2e6 rays, 24 parameters 0.70 -> 0.68 ms (0.69 with the
+// lanes made to meet first).
 template <class Sh>
-__device__ __forceinline__ void rev_surface(const AdjArgs& a, int k, RevRay& ray, int lane, double* acc_row) {
+__device__ __forceinline__ void rev_surface(const AdjArgs& a, int k, RevRay& ray, double* acc) {
     const DevScheme* sch = a.sch;
     const int np = a.surf_nparams[k];
     if (k == 0 && np == 0) return;  // the entrance rays' adjoint is not needed
@@ -231,34 +235,39 @@ __device__ __forceinline__ void rev_surface(const AdjArgs& a, int k, RevRay& ray
     if (ray.act) {
         const double* c = a.ckpt + (size_t)k * 6 * a.n + ray.i;
         const f64::Ray r0{c[0], c[a.n], c[2 * a.n], c[3 * a.n], c[4 * a.n], c[5 * a.n]};
-        if (!rv::surface_rev<Sh>(s, sch->fixes, a.knots, adj_order(s, a.beams, ray.b), ray.lam, r0, ray.adj, pa)) {
+        if (!rv::surface_rev<Sh>(s, sch->fixes, a.knots, adj_order(s, a.beams, ray.b), ray.lam, r0,
+                                 ray.have_out, ray.out, ray.adj, pa)) {
             ray.act = false;  // not reached: the recomputation is the forward's
-            rv::clear(pa);
         }
+        ray.out = r0;
     }
-    for (int q = 0; q < np; ++q) {
-        const int j = a.surf_params[k * RTB_ADJ_MAX_PARAMS + q];
-        double v = ray.act ? rv::param_adjoint(s, a.map[j], pa) : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) acc_row[j] += v;
+    ray.have_out = true;
+    if (ray.act) {
+        for (int q = 0; q < np; ++q) {
+            const int j = a.surf_params[k * RTB_ADJ_MAX_PARAMS + q];
+            acc[j * kAdjThreads] += rv::param_adjoint(s, a.map[j], pa);
+        }
     }
 }
 
 // The surfaces of any scheme, last to first, their structure read at run time.
 struct RtAdjSurfaces {
-    __device__ __forceinline__ static void sweep(const AdjArgs& a, RevRay& ray, int lane, double* acc_row) {
-        for (int k = a.sch->n_surfaces - 1; k >= 0; --k) rev_surface<RtShape>(a, k, ray, lane, acc_row);
+    __device__ __forceinline__ static void sweep(const AdjArgs& a, RevRay& ray, double* acc) {
+        for (int k = a.sch->n_surfaces - 1; k >= 0; --k) rev_surface<RtShape>(a, k, ray, acc);
     }
 };
 
-// gX, gY: the adjoints of the rays' CCD positions; partial: [gridDim.x][n_params].
+// gX, gY: the adjoints of the rays' CCD positions; partial: [gridDim.x][n_params];
+// dynamic shared memory: adj_reverse_smem(n_params).
+__host__ __device__ constexpr size_t adj_reverse_smem(int n_params) {
+    return (size_t)n_params * kAdjThreads * sizeof(double);
+}
 template <class Surfaces>
 __device__ __forceinline__ void adj_reverse(const AdjArgs& a, const double* gX, const double* gY, double* partial) {
-    __shared__ double acc[kAdjWarps][RTB_ADJ_MAX_PARAMS];
+    extern __shared__ double acc[];  // [n_params][kAdjThreads]
     const int P = a.n_params;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int p = lane; p < P; p += 32) acc[warp][p] = 0.0;
-    __syncwarp();
+    for (int p = 0; p < P; ++p) acc[p * kAdjThreads + threadIdx.x] = 0.0;
     for (size_t i0 = (size_t)blockIdx.x * blockDim.x + (size_t)warp * 32; i0 < a.n; i0 += gstride()) {
         RevRay ray;
         ray.i = i0 + lane;
@@ -268,13 +277,15 @@ __device__ __forceinline__ void adj_reverse(const AdjArgs& a, const double* gX, 
         if (!__any_sync(0xffffffffu, ray.act)) continue;
         ray.lam = ray.act ? a.lambda[ray.i] : 0.0;
         ray.b = ray.act ? beam_of(a.beams, a.n_beams, ray.i) : 0;
-        Surfaces::sweep(a, ray, lane, acc[warp]);
+        ray.have_out = false;
+        Surfaces::sweep(a, ray, acc + threadIdx.x);
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
+    for (int p = warp; p < P; p += kAdjWarps) {
         double sum = 0.0;
-        for (int w = 0; w < kAdjWarps; ++w) sum += acc[w][p];
-        partial[(size_t)blockIdx.x * P + p] = sum;
+        for (int w = 0; w < kAdjWarps; ++w) sum += acc[p * kAdjThreads + w * 32 + lane];
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) partial[(size_t)blockIdx.x * P + p] = sum;
     }
 }
 

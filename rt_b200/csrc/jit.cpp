@@ -445,9 +445,9 @@ std::string adjoint_source(const DevScheme& sch) {
         src += "        jvp_surface<" + adj_shape(sch.s[k]) + ">(a, " + std::to_string(k) + ", table, b, lam, r);\n";
     src += "    }\n};\n"
            "struct SchemeAdjSurfaces {\n"
-           "    __device__ __forceinline__ static void sweep(const AdjArgs& a, RevRay& ray, int lane, double* acc_row) {\n";
+           "    __device__ __forceinline__ static void sweep(const AdjArgs& a, RevRay& ray, double* acc) {\n";
     for (int k = sch.n_surfaces - 1; k >= 0; --k)
-        src += "        rev_surface<" + adj_shape(sch.s[k]) + ">(a, " + std::to_string(k) + ", ray, lane, acc_row);\n";
+        src += "        rev_surface<" + adj_shape(sch.s[k]) + ">(a, " + std::to_string(k) + ", ray, acc);\n";
     src += std::string("    }\n};\n}  // namespace rtb\n"
                        "extern \"C\" __global__ void __launch_bounds__(rtb::kAdjForwardThreads, 4) ") + kAdjForwardName +
            "(rtb::AdjArgs a, rtb::DevRays in,\n        unsigned long long* counts, unsigned* err) {\n"

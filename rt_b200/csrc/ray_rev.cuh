@@ -1,16 +1,17 @@
 // ray_rev.cuh -- reverse-mode derivatives of one surface of the plain FP64
 // engine.
 //
-// surface_rev recomputes a surface on one ray from the ray's state at the
-// surface's input (transform, normalise, and for a non-Aux surface the
-// intersection, action and second normalisation, with the plain engine's
-// functions and hence its values and branches), then carries the adjoint of
+// surface_rev takes a ray's states at the surface's input and output, restores
+// what lies between (transform, normalise, and for a non-Aux surface the point
+// of intersection, which is the output's position), and carries the adjoint of
 // the output state back through each stage in reverse order: the adjoint of
 // the input state and of the surface's differentiable constants (curvature,
 // conic constant, polynomial coefficients, toric radius, grating constant,
-// distances, rotation sines and cosines).  One recomputation and one reverse
-// sweep give every direction at once, where the forward-mode dual numbers of
-// ray_ad.cuh need one pass per few directions.
+// distances, rotation sines and cosines).  One reverse sweep gives every
+// direction at once, where the forward-mode dual numbers of ray_ad.cuh need
+// one pass per few directions.  Where the output state is not kept (the last
+// surface), the intersection and the action are recomputed with the plain
+// engine's functions.
 //
 // Each stage's adjoint is the transpose of the derivative ray_ad.cuh's dual
 // numbers compute for the same expression, so the two agree to rounding:
@@ -22,8 +23,8 @@
 //    distance) is the identity, whose derivative in its angle or distance is
 //    still taken.
 //
-// The translation unit is compiled with --fmad=false (the recomputed values
-// are the plain engine's bits).
+// The translation unit is compiled with --fmad=false (the plain engine's
+// functions have its bits).
 #pragma once
 
 #include "ray_ad.cuh"
@@ -33,9 +34,8 @@
 namespace rtb {
 namespace rv {
 
-// Reciprocal and reciprocal square root for the derivative arithmetic (the
-// values the recomputation follows keep the plain engine's IEEE operations):
-// the hardware seed refined by Newton steps (two for 1/x, x (2 - x y); two
+// Reciprocal and reciprocal square root for the derivative arithmetic: the
+// hardware seed refined by Newton steps (two for 1/x, x (2 - x y); two
 // for 1/sqrt(x), y (3/2 - x y^2 / 2)), to about an ulp, in place of the
 // IEEE division and square-root sequences.
 __device__ __forceinline__ double rcp(double x) { return ad::tangent_rcp(x); }
@@ -631,27 +631,48 @@ __device__ __forceinline__ void action_rev(const DevSurface& s, double mu, doubl
 
 // ---- one surface -----------------------------------------------------------------
 
-// Surface s on one ray from its input state r0: in, the adjoint of the
-// surface's output state; out, the adjoint of its input state, with the
-// constants' adjoints added to p.  False if the recomputation loses the ray
-// (it does not for a ray the forward traced through).
+// Surface s on one ray from its input state r0 and, with have_out, its output
+// state: in, the adjoint of the output state; out, the adjoint of the input
+// state, with the constants' adjoints added to p.  False if a recomputation
+// without the output loses the ray (it does not for a ray the forward traced
+// through).  The output's position is the point of intersection the forward
+// reported, so no root is found again and no branch taken anew; its cosines
+// are the action's result to rounding, which is a unit vector for every action
+// but a toric grating's, whose length the normalisation's adjoint needs.
 template <class Sh = RtShape>
 __device__ __forceinline__ bool surface_rev(const DevSurface& s, uint32_t fixes, const double* knots,
-                                            long long order, double lambda, const f64::Ray& r0, RayA& a,
-                                            SurfA& p) {
+                                            long long order, double lambda, const f64::Ray& r0, bool have_out,
+                                            const f64::Ray& out, RayA& a, SurfA& p) {
     f64::Ray r1 = r0;
     f64::transform<Sh>(s, r1);
     f64::Ray r2 = r1;
-    f64::normalize(r2.cX, r2.cY, r2.cZ);
+    const double in = rsqrt(fma(r1.cX, r1.cX, fma(r1.cY, r1.cY, r1.cZ * r1.cZ)));
+    r2.cX *= in;
+    r2.cY *= in;
+    r2.cZ *= in;
     if (Sh::non_aux(s)) {
         f64::Ray r3 = r2;
         double t;
-        if (!isect_fwd<Sh>(s, fixes, r3, t)) return false;
+        if (have_out) {
+            r3.X = out.X;
+            r3.Y = out.Y;
+            r3.Z = out.Z;
+            t = fma(r3.X - r2.X, r2.cX, fma(r3.Y - r2.Y, r2.cY, (r3.Z - r2.Z) * r2.cZ));
+        } else if (!isect_fwd<Sh>(s, fixes, r3, t)) {
+            return false;
+        }
         double mu, L;
         if (!action_consts<Sh>(s, knots, order, lambda, mu, L)) return false;
-        f64::Ray r4 = r3;
-        if (!action_fwd<Sh>(s, mu, L, r4)) return false;
-        normalize_rev(r4.cX, r4.cY, r4.cZ, a);
+        if (have_out && !(Sh::type(s) == RTB_GRATING && Sh::cls(s) == RTB_TORIC)) {
+            const double d = fma(a.cX, out.cX, fma(a.cY, out.cY, a.cZ * out.cZ));
+            a.cX = fma(-d, out.cX, a.cX);
+            a.cY = fma(-d, out.cY, a.cY);
+            a.cZ = fma(-d, out.cZ, a.cZ);
+        } else {
+            f64::Ray r4 = r3;
+            if (!action_fwd<Sh>(s, mu, L, r4)) return false;
+            normalize_rev(r4.cX, r4.cY, r4.cZ, a);
+        }
         action_rev<Sh>(s, mu, L, r3, a, p);
         isect_rev<Sh>(s, fixes, r2, t, a, p);
     }
