@@ -29,7 +29,7 @@ constexpr int kAdjWarps = kAdjThreads / 32;
 // does (C4, 2e6 rays: 0.36 ms, 0.38 at the 110 registers the compiler takes
 // unbounded); the reverse sweep at 128 and 16 warps (0.47; 0.60 at three
 // blocks an SM, 0.51 at five, where it spills); the sensitivities unbounded at
-// two blocks (0.88; 0.94 at the 128 registers of four).
+// two blocks (0.60; 0.94 against 0.87 at the 128 registers of four, before).
 constexpr int kAdjForwardThreads = 256;
 
 struct AdjArgs {

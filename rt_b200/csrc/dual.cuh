@@ -116,6 +116,15 @@ __device__ __forceinline__ double tangent_rcp(double x) {
     return fma(r, e, r);
 }
 
+// 1/sqrt(x) likewise: the hardware seed refined by two Newton steps.
+__device__ __forceinline__ double tangent_rsqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double h = 0.5 * x;
+    y = y * fma(-h * y, y, 1.5);
+    return y * fma(-h * y, y, 1.5);
+}
+
 template <int W>
 __device__ __forceinline__ Dual<W> operator/(const Dual<W>& a, const Dual<W>& b) {
     Dual<W> r;

@@ -39,13 +39,7 @@ namespace rv {
 // for 1/sqrt(x), y (3/2 - x y^2 / 2)), to about an ulp, in place of the
 // IEEE division and square-root sequences.
 __device__ __forceinline__ double rcp(double x) { return ad::tangent_rcp(x); }
-__device__ __forceinline__ double rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double h = 0.5 * x;
-    y = y * fma(-h * y, y, 1.5);
-    return y * fma(-h * y, y, 1.5);
-}
+__device__ __forceinline__ double rsqrt(double x) { return ad::tangent_rsqrt(x); }
 
 // Adjoints of the ray state.
 struct RayA {
