@@ -103,17 +103,6 @@ __global__ void k_build_surfd(AdjArgs a, const int2* entries, int n_entries, ad:
     ad::make_surfd(a.sch->s[k], k, a.map, a.n_params, sd, table[e]);
 }
 
-// The forward-mode constants of surface k along the direction dtheta.
-__global__ void k_build_surfd_dense(AdjArgs a, const double* dtheta, ad::SurfD<1>* table) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.sch->n_surfaces) return;
-    ad::Seeds<1> sd;
-    sd.dense = dtheta;
-    sd.state[0] = -1;
-    sd.param[0] = -1;
-    ad::make_surfd(a.sch->s[k], k, a.map, a.n_params, sd, table[k]);
-}
-
 // Rays are taken 32 at a time per warp, every lane of a warp the same number
 // of steps, so the warp can sum each parameter's contributions with shuffles.
 // first_entry[k]: the table entry of surface k's first pass.  Four blocks per
@@ -422,6 +411,20 @@ __global__ void __launch_bounds__(kMeritThreads) k_dense_seeds(const DenseBlock*
 
 using namespace rtb;
 
+namespace {
+// What the merits keep of a context's beams (MeritPass::make_plan): device
+// memory (from the pool: a first merit costs what a later one does) that holds
+// the groups or blocks, the partial sums and the seeds' coefficients.
+struct MeritPlan {
+    DevBuf buf;
+    char* mem = nullptr;  // set once all of it is there
+    bool dense = false;
+    int n_groups = 0;
+    unsigned n_blocks = 0;
+    size_t o_dgroups = 0, o_part = 0, o_coef = 0;
+};
+}  // namespace
+
 struct rtb_adjoint {
     int device = 0;
     std::vector<rtb_surface> surf;                 // the scheme, tables repointed to...
@@ -433,6 +436,7 @@ struct rtb_adjoint {
     uint64_t n = 0;
     uint32_t fixes = 0;
     PreparedScheme ps;
+    std::vector<ad::ParamRef> map;                 // the parameters by surface field
     bool have_forward = false;
     const void* fwd_kernel = nullptr;              // the forward, the reverse sweep and the
     const void* rev_kernel = nullptr;              // sensitivities compiled for the scheme's
@@ -454,8 +458,11 @@ struct rtb_adjoint {
     unsigned long long* d_counts = nullptr;
     unsigned* d_err = nullptr;
     double* d_grad = nullptr;
-    double* d_dtheta = nullptr;
+    ad::SurfD<1>* d_surfd = nullptr;               // the sensitivities' surface constants
     cudaStream_t stream = nullptr;
+    // the merits' groups and blocks, which follow from the beams: made and
+    // uploaded by the first merit
+    MeritPlan merit;
 };
 
 namespace {
@@ -564,6 +571,8 @@ AdjArgs adj_args(const rtb_adjoint* c) {
     a.flag = c->d_flag;
     a.X = c->d_X;
     a.Y = c->d_Y;
+    a.out_X = a.out_Y = nullptr;
+    a.out_flag = nullptr;
     a.n = c->n;
     return a;
 }
@@ -613,22 +622,24 @@ int rtb_adjoint_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb
         sp[p.surface * RTB_ADJ_MAX_PARAMS + sn[p.surface]++] = (int)j;
     }
     c->surf_nparams = sn;
-    // one allocation: scheme, knots (room for the largest table set), beams,
-    // map, lists, counters, grad; then the per-ray arrays
+    c->map = map;
+    // one allocation: scheme and knots (one upload of a forward), beams, map,
+    // lists, counters and error word (one memset, one copy back), grad; then
+    // the per-ray arrays
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
     c->knots_cap = c->ps.knots.size();
     const size_t ns1 = 3 * n_surfaces + 1;
     size_t off = 0;
-    const size_t o_sch = off; off += al(sizeof(DevScheme));
-    const size_t o_kn = off; off += al(c->knots_cap * sizeof(double));
+    const size_t o_sch = off; off += scheme_bytes((int)n_surfaces);
+    const size_t o_kn = off; off = al(off + c->knots_cap * sizeof(double));
     const size_t o_bm = off; off += al(n_beams * sizeof(DevBeam));
     const size_t o_map = off; off += al(map.size() * sizeof(ad::ParamRef));
     const size_t o_sp = off; off += al(sp.size() * sizeof(int));
     const size_t o_sn = off; off += al(sn.size() * sizeof(int));
-    const size_t o_cnt = off; off += al(n_beams * ns1 * 8);
-    const size_t o_err = off; off += 256;
+    const size_t o_cnt = off; off += al((n_beams * ns1 + 1) * 8);
+    const size_t o_err = o_cnt + n_beams * ns1 * 8;
     const size_t o_grad = off; off += al(RTB_ADJ_MAX_PARAMS * sizeof(double));
-    const size_t o_dth = off; off += al(RTB_ADJ_MAX_PARAMS * sizeof(double));
+    const size_t o_surfd = off; off += al(n_surfaces * sizeof(ad::SurfD<1>));
     const size_t o_ck = off; off += al(n_rays * 6 * n_surfaces * sizeof(double));
     const size_t o_lam = off; off += al(n_rays * sizeof(double));
     const size_t o_x = off; off += al(n_rays * sizeof(double));
@@ -651,7 +662,7 @@ int rtb_adjoint_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb
     c->d_counts = reinterpret_cast<unsigned long long*>(b + o_cnt);
     c->d_err = reinterpret_cast<unsigned*>(b + o_err);
     c->d_grad = reinterpret_cast<double*>(b + o_grad);
-    c->d_dtheta = reinterpret_cast<double*>(b + o_dth);
+    c->d_surfd = reinterpret_cast<ad::SurfD<1>*>(b + o_surfd);
     c->d_ckpt = reinterpret_cast<double*>(b + o_ck);
     c->d_lambda = reinterpret_cast<double*>(b + o_lam);
     c->d_X = reinterpret_cast<double*>(b + o_x);
@@ -716,12 +727,16 @@ int rtb_adjoint_forward(rtb_adjoint* c, const double* theta, const rtb_rays* ray
     c->ps = ps;
     const size_t ns1 = 3 * sf.size() + 1;
     const size_t nb = c->beams_h.size();
-    RTB_CUDA_TRY(cudaMemcpyAsync(c->d_sch, &ps.sch, sizeof(DevScheme), cudaMemcpyHostToDevice, s));
-    RTB_CUDA_TRY(cudaMemcpyAsync(c->d_knots, ps.knots.data(), ps.knots.size() * sizeof(double), cudaMemcpyHostToDevice,
-                                 s));
-    RTB_CUDA_TRY(cudaMemsetAsync(c->d_counts, 0, nb * ns1 * 8, s));
-    RTB_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, 4, s));
+    const size_t sch_bytes = scheme_bytes(ps.sch.n_surfaces), knot_bytes = ps.knots.size() * sizeof(double);
+    std::vector<char> h(sch_bytes + knot_bytes);
+    std::memcpy(h.data(), &ps.sch, sch_bytes);
+    std::memcpy(h.data() + sch_bytes, ps.knots.data(), knot_bytes);
+    RTB_CUDA_TRY(cudaMemcpyAsync(c->d_sch, h.data(), h.size(), cudaMemcpyHostToDevice, s));
+    RTB_CUDA_TRY(cudaMemsetAsync(c->d_counts, 0, (nb * ns1 + 1) * 8, s));
     AdjArgs a = adj_args(c);
+    a.out_X = X;
+    a.out_Y = Y;
+    a.out_flag = flag;
     DevRays in = dev_rays(rays);
     if (c->fwd_kernel) {
         unsigned long long* counts = c->d_counts;
@@ -733,16 +748,11 @@ int rtb_adjoint_forward(rtb_adjoint* c, const double* theta, const rtb_rays* ray
         k_adj_forward<<<adj_grid(c->n, kAdjForwardThreads), kAdjForwardThreads, 0, s>>>(a, in, c->d_counts, c->d_err);
     }
     RTB_CUDA_TRY(cudaGetLastError());
-    if (X) RTB_CUDA_TRY(cudaMemcpyAsync(X, c->d_X, c->n * 8, cudaMemcpyDeviceToDevice, s));
-    if (Y) RTB_CUDA_TRY(cudaMemcpyAsync(Y, c->d_Y, c->n * 8, cudaMemcpyDeviceToDevice, s));
-    if (flag) RTB_CUDA_TRY(cudaMemcpyAsync(flag, c->d_flag, c->n, cudaMemcpyDeviceToDevice, s));
-    std::vector<unsigned long long> counts(nb * ns1);
-    unsigned err = 0;
+    std::vector<unsigned long long> counts(nb * ns1 + 1);  // and the error word
     RTB_CUDA_TRY(cudaMemcpyAsync(counts.data(), c->d_counts, counts.size() * 8, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaMemcpyAsync(&err, c->d_err, 4, cudaMemcpyDeviceToHost, s));
     RTB_CUDA_TRY(cudaStreamSynchronize(s));
     c->have_forward = true;
-    return trace_result(ps, counts.data(), err, (int)nb, stats);
+    return trace_result(ps, counts.data(), (unsigned)counts[nb * ns1], (int)nb, stats);
 }
 
 int rtb_adjoint_backward(rtb_adjoint* c, const double* gX, const double* gY, double* grad, void* stream) {
@@ -810,17 +820,18 @@ int rtb_adjoint_jvp(rtb_adjoint* c, const double* dtheta, double* dX, double* dY
     DeviceGuard dg(c->device);
     Lock l;
     cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-    std::vector<double> d(RTB_ADJ_MAX_PARAMS, 0.0);
-    for (size_t j = 0; j < c->params.size(); ++j) d[j] = dtheta[j];
-    RTB_CUDA_TRY(cudaMemcpyAsync(c->d_dtheta, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice, s));
     AdjArgs a = adj_args(c);
+    // the surfaces' forward-mode constants along the direction
     const int ns = (int)c->surf_nparams.size();
-    DevBuf table;
-    int st = table.alloc((size_t)ns * sizeof(ad::SurfD<1>), s);
-    if (st != RTB_OK) return st;
-    k_build_surfd_dense<<<(unsigned)((ns + 31) / 32), 32, 0, s>>>(a, c->d_dtheta, table.as<ad::SurfD<1>>());
-    RTB_CUDA_TRY(cudaGetLastError());
-    const ad::SurfD<1>* tab = table.as<ad::SurfD<1>>();
+    std::vector<ad::SurfD<1>> table(ns);
+    ad::Seeds<1> sd;
+    sd.dense = dtheta;
+    sd.state[0] = -1;
+    sd.param[0] = -1;
+    for (int k = 0; k < ns; ++k)
+        ad::make_surfd(c->ps.sch.s[k], k, c->map.data(), (int)c->params.size(), sd, table[k]);
+    RTB_CUDA_TRY(cudaMemcpyAsync(c->d_surfd, table.data(), ns * sizeof(ad::SurfD<1>), cudaMemcpyHostToDevice, s));
+    const ad::SurfD<1>* tab = c->d_surfd;
     if (c->jvp_kernel) {
         void* args[] = {&a, &tab, &dX, &dY};
         RTB_CUDA_TRY(cudaLaunchKernel(c->jvp_kernel, dim3(adj_grid(c->n, kAdjThreads)), dim3(kAdjThreads), args, 0, s));
@@ -848,53 +859,22 @@ class MeritPass {
     MeritPass(rtb_adjoint* c, cudaStream_t s) : c_(c), s_(s) {}
 
     int moments(GroupMoments& m) {
-        for (const auto& b : c_->beams_in) {
-            const uint64_t nl = b.n_lambda ? b.n_lambda : 1;
-            for (uint64_t j = 0; j < nl; ++j) {
-                const uint64_t cnt = (b.n_rays > j) ? (b.n_rays - j + nl - 1) / nl : 0;
-                groups_.push_back(Group{b.first_ray + j, nl, cnt});
-            }
+        MeritPlan& mp = c_->merit;
+        if (!mp.mem) {
+            const int st = make_plan(mp);
+            if (st != RTB_OK) return st;
         }
-        G_ = (int)groups_.size();
-        if (G_ == 0 || G_ > 65535) return RTB_BAD_VALUE;
-        // index-order (dense) path: every beam of at most kMeritThreads wavelengths
-        dense_ = true;
-        for (const auto& b : c_->beams_in) dense_ = dense_ && (b.n_lambda ? b.n_lambda : 1) <= (uint64_t)kMeritThreads;
-        if (dense_) {
-            constexpr uint64_t kRaysPerThread = 8;
-            uint64_t pbase = 0;
-            int32_t gbase = 0;
-            for (const auto& b : c_->beams_in) {
-                const int32_t nl = (int32_t)(b.n_lambda ? b.n_lambda : 1);
-                const int32_t width = nl * (kMeritThreads / nl);
-                const uint64_t chunk = (uint64_t)width * kRaysPerThread;
-                const uint64_t nblk = (b.n_rays + chunk - 1) / chunk;
-                for (uint64_t k = 0; k < nblk; ++k) {
-                    const uint64_t start = b.first_ray + k * chunk;
-                    const uint64_t end = std::min(b.first_ray + b.n_rays, start + chunk);
-                    dblocks_.push_back(DenseBlock{start, end, nl, width, gbase, (int32_t)(pbase + k * (uint64_t)nl)});
-                }
-                for (int32_t j = 0; j < nl; ++j) dgroups_.push_back(DenseGroup{(int32_t)pbase, nl, (int32_t)nblk, j});
-                pbase += nblk * (uint64_t)nl;
-                gbase += nl;
-                if (pbase > (uint64_t)INT32_MAX || dblocks_.size() > (size_t)INT32_MAX) dense_ = false;
-            }
-        }
-        const size_t n_part = dense_ ? (size_t)dgroups_.back().pbase + (size_t)dgroups_.back().n_blocks * dgroups_.back().nl
-                                     : (size_t)G_ * kMeritParts;
-        const size_t tab_bytes = dense_ ? a256(dblocks_.size() * sizeof(DenseBlock)) + a256(G_ * sizeof(DenseGroup))
-                                        : a256(G_ * sizeof(Group));
-        const size_t part_bytes = a256(n_part * 3 * sizeof(double));
-        int st = buf_.alloc(tab_bytes + part_bytes + (size_t)G_ * (kSeedCoef + 2 + 6) * sizeof(double), s_);
-        if (st != RTB_OK) return st;
-        char* p = buf_.as<char>();
-        d_groups_ = reinterpret_cast<Group*>(p);
-        d_blocks_ = reinterpret_cast<DenseBlock*>(p);
-        DenseGroup* d_dgroups = reinterpret_cast<DenseGroup*>(p + a256(dblocks_.size() * sizeof(DenseBlock)));
-        double* d_part = reinterpret_cast<double*>(p + tab_bytes);
-        d_coef_ = reinterpret_cast<double*>(p + tab_bytes + part_bytes);  // kSeedCoef G
-        double* d_cen = d_coef_ + (size_t)kSeedCoef * G_;                    // 2 G
-        double* d_out = d_cen + 2 * (size_t)G_;                              // 6 G
+        G_ = mp.n_groups;
+        dense_ = mp.dense;
+        const unsigned n_blocks = mp.n_blocks;
+        d_groups_ = reinterpret_cast<Group*>(mp.mem);
+        d_blocks_ = reinterpret_cast<DenseBlock*>(mp.mem);
+        DenseGroup* d_dgroups = reinterpret_cast<DenseGroup*>(mp.mem + mp.o_dgroups);
+        double* d_part = reinterpret_cast<double*>(mp.mem + mp.o_part);
+        d_coef_ = reinterpret_cast<double*>(mp.mem + mp.o_coef);  // kSeedCoef G
+        double* d_cen = d_coef_ + (size_t)kSeedCoef * G_;           // 2 G
+        double* d_out = d_cen + 2 * (size_t)G_;                     // 6 G
+        n_blocks_ = n_blocks;
         m.n.assign(G_, 0.0);
         m.cx.assign(G_, 0.0);
         m.cy.assign(G_, 0.0);
@@ -903,14 +883,10 @@ class MeritPass {
         m.sxy.assign(G_, 0.0);
         cudaStream_t s = s_;
         if (dense_) {
-            if (!dblocks_.empty())
-                RTB_CUDA_TRY(cudaMemcpyAsync(d_blocks_, dblocks_.data(), dblocks_.size() * sizeof(DenseBlock),
-                                             cudaMemcpyHostToDevice, s));
-            RTB_CUDA_TRY(cudaMemcpyAsync(d_dgroups, dgroups_.data(), G_ * sizeof(DenseGroup), cudaMemcpyHostToDevice, s));
             for (int pass = 0; pass < 2; ++pass) {
-                if (!dblocks_.empty())
-                    k_dense_moments<<<(unsigned)dblocks_.size(), kMeritThreads, 0, s>>>(d_blocks_, c_->d_flag, c_->d_X,
-                                                                                        c_->d_Y, d_cen, pass, d_part);
+                if (n_blocks)
+                    k_dense_moments<<<n_blocks, kMeritThreads, 0, s>>>(d_blocks_, c_->d_flag, c_->d_X, c_->d_Y, d_cen,
+                                                                       pass, d_part);
                 k_dense_finish<<<G_, kMeritThreads, 0, s>>>(d_dgroups, d_part, pass, d_cen, d_out);
                 RTB_CUDA_TRY(cudaGetLastError());
             }
@@ -927,7 +903,6 @@ class MeritPass {
             }
             return RTB_OK;
         }
-        RTB_CUDA_TRY(cudaMemcpyAsync(d_groups_, groups_.data(), G_ * sizeof(Group), cudaMemcpyHostToDevice, s));
         std::vector<double> part((size_t)G_ * kMeritParts * 3), cen(2 * (size_t)G_);
         for (int pass = 0; pass < 2; ++pass) {
             if (pass == 1)
@@ -976,9 +951,9 @@ class MeritPass {
         RTB_CUDA_TRY(zero(from, c_->n));
         RTB_CUDA_TRY(cudaMemcpyAsync(d_coef_, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, s));
         if (dense_) {
-            if (!dblocks_.empty())
-                k_dense_seeds<<<(unsigned)dblocks_.size(), kMeritThreads, 0, s>>>(d_blocks_, d_coef_, c_->d_flag,
-                                                                                  c_->d_X, c_->d_Y, gX, gY);
+            if (n_blocks_)
+                k_dense_seeds<<<n_blocks_, kMeritThreads, 0, s>>>(d_blocks_, d_coef_, c_->d_flag, c_->d_X, c_->d_Y, gX,
+                                                                  gY);
         } else {
             k_group_seeds<<<dim3(G_, 64), 256, 0, s>>>(d_groups_, G_, d_coef_, c_->d_flag, c_->d_X, c_->d_Y, gX, gY);
         }
@@ -991,14 +966,81 @@ class MeritPass {
 
   private:
     static size_t a256(size_t b) { return (b + 255) / 256 * 256; }
+
+    // Groups, and for beams of few wavelengths the blocks in index order, on
+    // the device with the room the moments need.
+    int make_plan(MeritPlan& mp) {
+        std::vector<Group> groups;
+        std::vector<DenseBlock> dblocks;
+        std::vector<DenseGroup> dgroups;
+        for (const auto& b : c_->beams_in) {
+            const uint64_t nl = b.n_lambda ? b.n_lambda : 1;
+            for (uint64_t j = 0; j < nl; ++j) {
+                const uint64_t cnt = (b.n_rays > j) ? (b.n_rays - j + nl - 1) / nl : 0;
+                groups.push_back(Group{b.first_ray + j, nl, cnt});
+            }
+        }
+        const size_t G = groups.size();
+        if (G == 0 || G > 65535) return RTB_BAD_VALUE;
+        // index-order (dense) path: every beam of at most kMeritThreads wavelengths
+        bool dense = true;
+        for (const auto& b : c_->beams_in) dense = dense && (b.n_lambda ? b.n_lambda : 1) <= (uint64_t)kMeritThreads;
+        if (dense) {
+            constexpr uint64_t kRaysPerThread = 8;
+            uint64_t pbase = 0;
+            int32_t gbase = 0;
+            for (const auto& b : c_->beams_in) {
+                const int32_t nl = (int32_t)(b.n_lambda ? b.n_lambda : 1);
+                const int32_t width = nl * (kMeritThreads / nl);
+                const uint64_t chunk = (uint64_t)width * kRaysPerThread;
+                const uint64_t nblk = (b.n_rays + chunk - 1) / chunk;
+                for (uint64_t k = 0; k < nblk; ++k) {
+                    const uint64_t start = b.first_ray + k * chunk;
+                    const uint64_t end = std::min(b.first_ray + b.n_rays, start + chunk);
+                    dblocks.push_back(DenseBlock{start, end, nl, width, gbase, (int32_t)(pbase + k * (uint64_t)nl)});
+                }
+                for (int32_t j = 0; j < nl; ++j) dgroups.push_back(DenseGroup{(int32_t)pbase, nl, (int32_t)nblk, j});
+                pbase += nblk * (uint64_t)nl;
+                gbase += nl;
+                if (pbase > (uint64_t)INT32_MAX || dblocks.size() > (size_t)INT32_MAX) dense = false;
+            }
+        }
+        const size_t n_part = dense ? (size_t)dgroups.back().pbase + (size_t)dgroups.back().n_blocks * dgroups.back().nl
+                                    : G * kMeritParts;
+        mp.dense = dense;
+        mp.n_groups = (int)G;
+        mp.n_blocks = dense ? (unsigned)dblocks.size() : 0;
+        mp.o_dgroups = dense ? a256(dblocks.size() * sizeof(DenseBlock)) : 0;
+        mp.o_part = mp.o_dgroups + (dense ? a256(G * sizeof(DenseGroup)) : a256(G * sizeof(Group)));
+        mp.o_coef = mp.o_part + a256(n_part * 3 * sizeof(double));
+        const int st = mp.buf.alloc(mp.o_coef + G * (kSeedCoef + 2 + 6) * sizeof(double), s_);
+        if (st != RTB_OK) return st;
+        char* mem = mp.buf.as<char>();
+        cudaError_t e = cudaSuccess;
+        if (dense) {
+            if (!dblocks.empty())
+                e = cudaMemcpyAsync(mem, dblocks.data(), dblocks.size() * sizeof(DenseBlock), cudaMemcpyHostToDevice, s_);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(mem + mp.o_dgroups, dgroups.data(), G * sizeof(DenseGroup), cudaMemcpyHostToDevice,
+                                    s_);
+        } else {
+            e = cudaMemcpyAsync(mem, groups.data(), G * sizeof(Group), cudaMemcpyHostToDevice, s_);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
+        if (e != cudaSuccess) {
+            mp.buf.release();
+            return cuda_status(e);
+        }
+        mp.buf.s = c_->stream;  // freed there: the caller's stream may be gone by then
+        mp.mem = mem;
+        return RTB_OK;
+    }
+
     rtb_adjoint* c_;
     cudaStream_t s_;
-    std::vector<Group> groups_;
-    std::vector<DenseBlock> dblocks_;
-    std::vector<DenseGroup> dgroups_;
     int G_ = 0;
     bool dense_ = false;
-    DevBuf buf_;
+    unsigned n_blocks_ = 0;
     Group* d_groups_ = nullptr;
     DenseBlock* d_blocks_ = nullptr;
     double* d_coef_ = nullptr;
@@ -1110,6 +1152,8 @@ int rtb_adjoint_resolution_merit(rtb_adjoint* c, const double* lambda, double ux
 int rtb_adjoint_destroy(rtb_adjoint* c) {
     if (!c) return RTB_OK;
     DeviceGuard dg(c->device);
+    if (c->stream) cudaStreamSynchronize(c->stream);
+    c->merit.buf.release();
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->mem) cudaFree(c->mem);
     if (c->stream) cudaStreamDestroy(c->stream);

@@ -46,6 +46,10 @@ struct AdjArgs {
     char* flag;              // 1 = reached the end
     double* X;
     double* Y;
+    // the forward's caller's copies of X, Y and flag, each may be NULL
+    double* out_X;
+    double* out_Y;
+    char* out_flag;
     uint64_t n;
 };
 
@@ -156,7 +160,13 @@ __device__ __forceinline__ void adj_forward(const AdjArgs& a, const DevRays& in,
             a.Y[i] = r.Y;
         }
         __syncwarp();
-        if (i < a.n) a.flag[i] = (stage == -1) ? 1 : 0;
+        if (i < a.n) {
+            const char f = (stage == -1) ? 1 : 0;
+            a.flag[i] = f;
+            if (a.out_flag) a.out_flag[i] = f;
+            if (a.out_X) a.out_X[i] = a.X[i];
+            if (a.out_Y) a.out_Y[i] = a.Y[i];
+        }
         // one atomic per distinct counter in the warp (the rays of a beam
         // mostly share theirs)
         count_event(stage != -2, b * (n_stages + 1) + (stage >= 0 ? stage : n_stages), counts);

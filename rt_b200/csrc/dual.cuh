@@ -22,7 +22,7 @@ struct Dual {
 };
 
 template <int W>
-__device__ __forceinline__ Dual<W> cst(double v) {
+__host__ __device__ __forceinline__ Dual<W> cst(double v) {
     Dual<W> r;
     r.v = v;
 #pragma unroll

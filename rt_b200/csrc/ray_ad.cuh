@@ -59,12 +59,12 @@ struct Seeds {
 };
 
 template <int W>
-__device__ __forceinline__ void seed_field(Dual<W>& f, int lane, double w) {
+__host__ __device__ __forceinline__ void seed_field(Dual<W>& f, int lane, double w) {
     f.d[lane] += w;
 }
 
 template <int W>
-__device__ void make_surfd(const DevSurface& s, int k, const ParamRef* map, int n_params, const Seeds<W>& sd,
+__host__ __device__ inline void make_surfd(const DevSurface& s, int k, const ParamRef* map, int n_params, const Seeds<W>& sd,
                            SurfD<W>& o) {
     o.c = cst<W>(s.c);
     o.k1 = cst<W>(s.k1);
