@@ -11,6 +11,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 
 #include "engine.cuh"
@@ -450,31 +452,106 @@ static void spline_second_derivatives(size_t N, const double* x, const double* y
 // ---------------------------------------------------------------------------
 // Drop-in helpers
 
+// Page-locked host vectors the library handed out (rtb_alocate_vector), by
+// address: the device reads and writes them in place.
+static std::mutex g_vectors_mu;
+static std::map<uintptr_t, size_t> g_vectors;
+
+bool in_host_vector(const void* p, size_t bytes) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    std::lock_guard<std::mutex> g(g_vectors_mu);
+    auto it = g_vectors.upper_bound(at);
+    if (it == g_vectors.begin()) return false;
+    --it;
+    return at - it->first <= it->second && bytes <= it->second - (at - it->first);
+}
+
 namespace {
 
-// Device copies of up to 8 double arrays and one flag array, from one pool
-// allocation.
-struct Staged {
+// The host arrays of one drop-in call as its kernel sees them.  An array in a
+// library vector is passed to the kernel as it is: the kernel's loads and
+// stores cross the link in both directions at once, where copies of each array
+// before and after it went one by one, some nine calls of a few microseconds
+// and as many transfers (C0's four surfaces on 1e5 rays, 29 calls: 3.7 ms of
+// copies and kernels on the device, 2.1 now).  Other arrays (the reference allocates Beam::flag with new[]) are
+// copied to the device and back.  The counter of lost rays and the error word
+// are at the start of the one pool allocation.
+struct HostArrays {
+    static constexpr int kMax = 9;
+    struct Entry {
+        void* host;
+        void* dev;
+        size_t bytes;
+        bool in, out, staged;
+    } e[kMax];
+    int n = 0;
     DevBuf buf;
-    double* d[8] = {nullptr};
-    char* flag = nullptr;
     unsigned long long* counter = nullptr;
     unsigned* err = nullptr;
-    int init(size_t n, int n_double, bool with_flag, cudaStream_t st) {
-        size_t bytes = 64 + n_double * n * sizeof(double) + (with_flag ? n + 16 : 0);
+    cudaStream_t st;
+    explicit HostArrays(cudaStream_t s) : st(s) {}
+    void add(const void* host, size_t bytes, bool in, bool out) {
+        const bool staged = !in_host_vector(host, bytes);
+        e[n++] = Entry{const_cast<void*>(host), staged ? nullptr : const_cast<void*>(host), bytes, in, out, staged};
+    }
+    int open(bool counted) {
+        // arrays that share memory are copied, so that each is read as it was
+        for (int i = 0; i < n; ++i)
+            for (int j = 0; j < n; ++j) {
+                const char *a = static_cast<const char*>(e[i].host), *b = static_cast<const char*>(e[j].host);
+                if (i != j && a < b + e[j].bytes && b < a + e[i].bytes) e[i].staged = true;
+            }
+        size_t bytes = counted ? 64 : 0;
+        for (int i = 0; i < n; ++i)
+            if (e[i].staged) bytes += (e[i].bytes + 15) / 16 * 16;
+        if (bytes == 0) return RTB_OK;
         int s = buf.alloc(bytes, st);
         if (s != RTB_OK) return s;
         char* p = buf.as<char>();
-        counter = reinterpret_cast<unsigned long long*>(p);
-        err = reinterpret_cast<unsigned*>(p + 8);
-        p += 64;
-        for (int i = 0; i < n_double; ++i) {
-            d[i] = reinterpret_cast<double*>(p);
-            p += n * sizeof(double);
+        if (counted) {
+            counter = reinterpret_cast<unsigned long long*>(p);
+            err = reinterpret_cast<unsigned*>(p + 8);
+            RTB_CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
+            p += 64;
         }
-        if (with_flag) flag = p;
-        RTB_CUDA_TRY(cudaMemsetAsync(buf.p, 0, 64, st));
+        for (int i = 0; i < n; ++i) {
+            if (!e[i].staged) continue;
+            e[i].dev = p;
+            p += (e[i].bytes + 15) / 16 * 16;
+            if (e[i].in) RTB_CUDA_TRY(cudaMemcpyAsync(e[i].dev, e[i].host, e[i].bytes, cudaMemcpyHostToDevice, st));
+        }
         return RTB_OK;
+    }
+    // Copies back what was staged, waits, and adds the lost rays to *n_bad.
+    int close(size_t* n_bad = nullptr) {
+        RTB_CUDA_TRY(cudaGetLastError());
+        for (int i = 0; i < n; ++i)
+            if (e[i].staged && e[i].out)
+                RTB_CUDA_TRY(cudaMemcpyAsync(e[i].host, e[i].dev, e[i].bytes, cudaMemcpyDeviceToHost, st));
+        unsigned long long h[2] = {0, 0};
+        if (counter) RTB_CUDA_TRY(cudaMemcpyAsync(h, counter, sizeof(h), cudaMemcpyDeviceToHost, st));
+        RTB_CUDA_TRY(cudaStreamSynchronize(st));
+        RTB_CUDA_TRY(cudaGetLastError());
+        if ((unsigned)h[1] & DEV_ERR_OUT_OF_RANGE) return RTB_OUT_OF_RANGE;
+        if ((unsigned)h[1]) return RTB_BAD_VALUE;
+        if (n_bad) *n_bad += (size_t)h[0];
+        return RTB_OK;
+    }
+    // Blocks for a kernel over `count` rays.  Over the link few threads are
+    // enough to keep it busy, and with more of them all the loads go before
+    // all the stores, one direction at a time: the transform of 1e5 rays took
+    // 171 us with a thread per ray, 141 at 148 blocks, 126 at 16 to 48, 131 at 8.
+    static constexpr unsigned kLinkBlocks = 48;
+    unsigned grid(size_t count) const {
+        bool mapped = false;
+        for (int i = 0; i < n; ++i) mapped = mapped || !e[i].staged;
+        const unsigned b = grid_for(count, 256, 8);
+        return mapped && b > kLinkBlocks ? kLinkBlocks : b;
+    }
+    double* d(int i) const { return static_cast<double*>(e[i].dev); }
+    template <class T>
+    T* as(int i) const {
+        return static_cast<T*>(e[i].dev);
     }
 };
 
@@ -490,17 +567,13 @@ int d2h(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     return RTB_OK;
 }
 
-int finish(cudaStream_t st, const unsigned* d_err, size_t* n_bad, const unsigned long long* d_counter) {
-    unsigned long long cnt = 0;
+int finish(cudaStream_t st, const unsigned* d_err) {
     unsigned err = 0;
-    if (d_counter) RTB_CUDA_TRY(cudaMemcpyAsync(&cnt, d_counter, sizeof(cnt), cudaMemcpyDeviceToHost, st));
-    if (d_err) RTB_CUDA_TRY(cudaMemcpyAsync(&err, d_err, sizeof(err), cudaMemcpyDeviceToHost, st));
+    RTB_CUDA_TRY(cudaMemcpyAsync(&err, d_err, sizeof(err), cudaMemcpyDeviceToHost, st));
     RTB_CUDA_TRY(cudaStreamSynchronize(st));
     RTB_CUDA_TRY(cudaGetLastError());
     if (err & DEV_ERR_OUT_OF_RANGE) return RTB_OUT_OF_RANGE;
-    if (err) return RTB_BAD_VALUE;
-    if (n_bad) *n_bad += (size_t)cnt;
-    return RTB_OK;
+    return err ? RTB_BAD_VALUE : RTB_OK;
 }
 
 }  // namespace
@@ -547,13 +620,25 @@ int rtb_spline_init(size_t n, const double* x, const double* y, double* y2) {
 }
 
 double* rtb_alocate_vector(size_t n_elem) {
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(double) * (n_elem ? n_elem : 1), cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    void *p = nullptr, *d = nullptr;
+    const size_t bytes = sizeof(double) * (n_elem ? n_elem : 1);
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    if (cudaHostGetDevicePointer(&d, p, 0) == cudaSuccess && d == p) {  // one address on both sides (UVA)
+        std::lock_guard<std::mutex> g(g_vectors_mu);
+        g_vectors[reinterpret_cast<uintptr_t>(p)] = bytes;
+    } else {
+        cudaGetLastError();
+    }
     return static_cast<double*>(p);
 }
 
 void rtb_free_vector(double* data) {
-    if (data) cudaFreeHost(data);
+    if (!data) return;
+    {
+        std::lock_guard<std::mutex> g(g_vectors_mu);
+        g_vectors.erase(reinterpret_cast<uintptr_t>(data));
+    }
+    cudaFreeHost(data);
 }
 
 int rtb_beam_random(int shape, const double* params, const double* center, size_t n, double* X, double* Y, double* Z,
@@ -564,14 +649,12 @@ int rtb_beam_random(int shape, const double* params, const double* center, size_
     int st = ensure_init();
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 3, false, s)) != RTB_OK) return st;
-    k_beam_random<<<grid_for(n, 256, 8), 256, 0, s>>>(n, params[1], params[2], center[0], center[1], center[2], seed,
-                                                        first_ray, g.d[0], g.d[1], g.d[2]);
-    double* out[3] = {X, Y, Z};
-    for (int i = 0; i < 3; ++i)
-        if ((st = d2h(out[i], g.d[i], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), false, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_beam_random<<<g.grid(n), 256, 0, s>>>(n, params[1], params[2], center[0], center[1], center[2], seed,
+                                                        first_ray, g.d(0), g.d(1), g.d(2));
+    return g.close();
 }
 
 // conic_cosins_kernel (rt_cuda_engine_beam.cu:586-611): cZ = cos(a/2),
@@ -633,11 +716,11 @@ int rtb_uniform_range_beam(size_t n, const double* range, double* lambda) {
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     double d_l = (range[1] - range[0]) / (n - 1);  // rt_cuda_engine_beam.cu:726
-    Staged g;
-    if ((st = g.init(n, 1, false, s)) != RTB_OK) return st;
-    k_uniform_range<<<grid_for(n, 256, 8), 256, 0, s>>>(n, range[0], d_l, g.d[0]);
-    if ((st = d2h(lambda, g.d[0], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    g.add(lambda, n * sizeof(double), false, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_uniform_range<<<g.grid(n), 256, 0, s>>>(n, range[0], d_l, g.d(0));
+    return g.close();
 }
 
 int rtb_random_range_beam(size_t n, const double* range, double* lambda, uint64_t seed) {
@@ -647,11 +730,11 @@ int rtb_random_range_beam(size_t n, const double* range, double* lambda, uint64_
     int st = ensure_init();
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 1, false, s)) != RTB_OK) return st;
-    k_random_range<<<grid_for(n, 256, 8), 256, 0, s>>>(n, range[0], range[1], seed, g.d[0]);
-    if ((st = d2h(lambda, g.d[0], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    g.add(lambda, n * sizeof(double), false, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_random_range<<<g.grid(n), 256, 0, s>>>(n, range[0], range[1], seed, g.d(0));
+    return g.close();
 }
 
 int rtb_beam_transform(size_t n, const double* angles, const double* dist, double* X, double* Y, double* Z,
@@ -665,15 +748,11 @@ int rtb_beam_transform(size_t n, const double* angles, const double* dist, doubl
     DevSurface ds;
     std::memset(&ds, 0, sizeof(ds));
     transform_constants(angles, dist, ds);
-    Staged g;
-    if ((st = g.init(n, 6, false, s)) != RTB_OK) return st;
-    double* a[6] = {X, Y, Z, cX, cY, cZ};
-    for (int i = 0; i < 6; ++i)
-        if ((st = h2d(g.d[i], a[i], n * sizeof(double), s)) != RTB_OK) return st;
-    k_transform<<<grid_for(n, 256, 8), 256, 0, s>>>(n, ds, g.d[0], g.d[1], g.d[2], g.d[3], g.d[4], g.d[5]);
-    for (int i = 0; i < 6; ++i)
-        if ((st = d2h(a[i], g.d[i], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    for (double* p : {X, Y, Z, cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_transform<<<g.grid(n), 256, 0, s>>>(n, ds, g.d(0), g.d(1), g.d(2), g.d(3), g.d(4), g.d(5));
+    return g.close();
 }
 
 static int intersection_impl(int cls, const double* params, size_t n, double* X, double* Y, double* Z, double* cX,
@@ -686,18 +765,14 @@ static int intersection_impl(int cls, const double* params, size_t n, double* X,
     Lock l;
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 6, true, s)) != RTB_OK) return st;
-    double* a[6] = {X, Y, Z, cX, cY, cZ};
-    for (int i = 0; i < 6; ++i)
-        if ((st = h2d(g.d[i], a[i], n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.flag, flag, n, s)) != RTB_OK) return st;
-    k_intersect<<<grid_for(n, 256, 8), 256, 0, s>>>(n, ds, fixes, g.d[0], g.d[1], g.d[2], g.d[3], g.d[4], g.d[5],
-                                                      g.flag, g.counter);
-    for (int i = 0; i < 3; ++i)
-        if ((st = d2h(a[i], g.d[i], n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = d2h(flag, g.flag, n, s)) != RTB_OK) return st;
-    return finish(s, g.err, n_bad, g.counter);
+    HostArrays g(s);
+    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), true, true);
+    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, false);
+    g.add(flag, n, true, true);
+    if ((st = g.open(true)) != RTB_OK) return st;
+    k_intersect<<<g.grid(n), 256, 0, s>>>(n, ds, fixes, g.d(0), g.d(1), g.d(2), g.d(3), g.d(4), g.d(5),
+                                                      g.as<char>(6), g.counter);
+    return g.close(n_bad);
 }
 
 int rtb_surface_intersection(int cls, const double* params, size_t n, double* X, double* Y, double* Z, double* cX,
@@ -719,15 +794,12 @@ int rtb_surface_reflection(int cls, const double* params, size_t n, double* X, d
     Lock l;
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 6, false, s)) != RTB_OK) return st;
-    double* a[6] = {X, Y, Z, cX, cY, cZ};
-    for (int i = 0; i < 6; ++i)
-        if ((st = h2d(g.d[i], a[i], n * sizeof(double), s)) != RTB_OK) return st;
-    k_reflect<<<grid_for(n, 256, 8), 256, 0, s>>>(n, ds, g.d[0], g.d[1], g.d[2], g.d[3], g.d[4], g.d[5]);
-    for (int i = 3; i < 6; ++i)
-        if ((st = d2h(a[i], g.d[i], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), true, false);
+    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_reflect<<<g.grid(n), 256, 0, s>>>(n, ds, g.d(0), g.d(1), g.d(2), g.d(3), g.d(4), g.d(5));
+    return g.close();
 }
 
 // Refraction (type Lens) or diffraction (type Grating) over host arrays.
@@ -750,22 +822,16 @@ static int action_impl(int type, int cls, int gr_type, const double* params, lon
     Lock l;
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 7, true, s)) != RTB_OK) return st;
-    DevBuf kb;
-    if ((st = kb.alloc(knots.size() * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(kb.p, knots.data(), knots.size() * sizeof(double), s)) != RTB_OK) return st;
-    double* a[6] = {X, Y, Z, cX, cY, cZ};
-    for (int i = 0; i < 6; ++i)
-        if ((st = h2d(g.d[i], a[i], n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[6], lambda, n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.flag, flag, n, s)) != RTB_OK) return st;
-    k_action<<<grid_for(n, 256, 8), 256, 0, s>>>(n, ds, kb.as<double>(), (long long)order, g.d[6], g.d[0], g.d[1],
-                                                   g.d[2], g.d[3], g.d[4], g.d[5], g.flag, g.counter, g.err);
-    for (int i = 3; i < 6; ++i)
-        if ((st = d2h(a[i], g.d[i], n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = d2h(flag, g.flag, n, s)) != RTB_OK) return st;
-    return finish(s, g.err, n_bad, g.counter);
+    HostArrays g(s);
+    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), true, false);
+    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    g.add(lambda, n * sizeof(double), true, false);
+    g.add(flag, n, true, true);
+    g.add(knots.data(), knots.size() * sizeof(double), true, false);
+    if ((st = g.open(true)) != RTB_OK) return st;
+    k_action<<<g.grid(n), 256, 0, s>>>(n, ds, g.d(8), (long long)order, g.d(6), g.d(0), g.d(1), g.d(2), g.d(3),
+                                                   g.d(4), g.d(5), g.as<char>(7), g.counter, g.err);
+    return g.close(n_bad);
 }
 
 int rtb_surface_refraction(int cls, const double* params, size_t n, double* X, double* Y, double* Z, double* cX,
@@ -792,16 +858,13 @@ int rtb_surface_QE(size_t n, const double* lambda, double* spec, const rtb_table
     Lock l;
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 2, false, s)) != RTB_OK) return st;
-    DevBuf kb;
-    if ((st = kb.alloc(knots.size() * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(kb.p, knots.data(), knots.size() * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[0], lambda, n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[1], spec, n * sizeof(double), s)) != RTB_OK) return st;
-    k_surface_qe<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d[0], g.d[1], kb.as<double>(), off, cnt, g.err);
-    if ((st = d2h(spec, g.d[1], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, g.err, nullptr, nullptr);
+    HostArrays g(s);
+    g.add(lambda, n * sizeof(double), true, false);
+    g.add(spec, n * sizeof(double), true, true);
+    g.add(knots.data(), knots.size() * sizeof(double), true, false);
+    if ((st = g.open(true)) != RTB_OK) return st;
+    k_surface_qe<<<g.grid(n), 256, 0, s>>>(n, g.d(0), g.d(1), g.d(2), off, cnt, g.err);
+    return g.close();
 }
 
 int rtb_normalize(size_t n, double* cX, double* cY, double* cZ) {
@@ -810,15 +873,11 @@ int rtb_normalize(size_t n, double* cX, double* cY, double* cZ) {
     int st = ensure_init();
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 3, false, s)) != RTB_OK) return st;
-    double* a[3] = {cX, cY, cZ};
-    for (int i = 0; i < 3; ++i)
-        if ((st = h2d(g.d[i], a[i], n * sizeof(double), s)) != RTB_OK) return st;
-    k_normalize<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d[0], g.d[1], g.d[2]);
-    for (int i = 0; i < 3; ++i)
-        if ((st = d2h(a[i], g.d[i], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_normalize<<<g.grid(n), 256, 0, s>>>(n, g.d(0), g.d(1), g.d(2));
+    return g.close();
 }
 
 int rtb_apply_constrains(int shade, int shape, const double* size, const double* center, size_t n, const double* X,
@@ -830,15 +889,14 @@ int rtb_apply_constrains(int shade, int shape, const double* size, const double*
     int st = ensure_init();
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 2, true, s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[0], X, n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[1], Y, n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.flag, flag, n, s)) != RTB_OK) return st;
-    k_aperture<<<grid_for(n, 256, 8), 256, 0, s>>>(n, shade, shape, size[0], shape == RTB_RECTANGLE ? size[1] : 0.0,
-                                                     center[0], center[1], g.d[0], g.d[1], g.flag, g.counter);
-    if ((st = d2h(flag, g.flag, n, s)) != RTB_OK) return st;
-    return finish(s, nullptr, n_bad, g.counter);
+    HostArrays g(s);
+    g.add(X, n * sizeof(double), true, false);
+    g.add(Y, n * sizeof(double), true, false);
+    g.add(flag, n, true, true);
+    if ((st = g.open(true)) != RTB_OK) return st;
+    k_aperture<<<g.grid(n), 256, 0, s>>>(n, shade, shape, size[0], shape == RTB_RECTANGLE ? size[1] : 0.0,
+                                                     center[0], center[1], g.d(0), g.d(1), g.as<char>(2), g.counter);
+    return g.close(n_bad);
 }
 
 int rtb_ccd_coordinates(size_t n, const double* X, const double* Y, double xsize, double ysize, double xpix,
@@ -848,16 +906,15 @@ int rtb_ccd_coordinates(size_t n, const double* X, const double* Y, double xsize
     int st = ensure_init();
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 3, false, s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[0], X, n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[1], Y, n * sizeof(double), s)) != RTB_OK) return st;
-    unsigned* ix = reinterpret_cast<unsigned*>(g.d[2]);
-    unsigned* iy = ix + n;
-    k_ccd_coords<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d[0], g.d[1], xsize, ysize, xpix, ypix, ix, iy);
-    if ((st = d2h(ccd_X, ix, n * sizeof(unsigned), s)) != RTB_OK) return st;
-    if ((st = d2h(ccd_Y, iy, n * sizeof(unsigned), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    g.add(X, n * sizeof(double), true, false);
+    g.add(Y, n * sizeof(double), true, false);
+    g.add(ccd_X, n * sizeof(unsigned), false, true);
+    g.add(ccd_Y, n * sizeof(unsigned), false, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_ccd_coords<<<g.grid(n), 256, 0, s>>>(n, g.d(0), g.d(1), xsize, ysize, xpix, ypix, g.as<unsigned>(2),
+                                                       g.as<unsigned>(3));
+    return g.close();
 }
 
 int rtb_compute_ccd_image(size_t n, const unsigned int* ccd_X, const unsigned int* ccd_Y, const double* lambda,
@@ -874,26 +931,28 @@ int rtb_compute_ccd_image(size_t n, const unsigned int* ccd_X, const unsigned in
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     size_t npix = xdim * ydim;
-    DevBuf img, kb;
+    // the image's pixels are added to at random: it is worked on in device
+    // memory, the rays' arrays are read where they are
+    DevBuf img;
     if ((st = img.alloc(npix * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = kb.alloc(knots.size() * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(kb.p, knots.data(), knots.size() * sizeof(double), s)) != RTB_OK) return st;
     if ((st = h2d(img.p, image, npix * sizeof(double), s)) != RTB_OK) return st;
-    Staged g;
-    if ((st = g.init(n ? n : 1, 2, false, s)) != RTB_OK) return st;
+    HostArrays g(s);
+    g.add(knots.data(), knots.size() * sizeof(double), true, false);
     if (n) {
-        unsigned* ix = reinterpret_cast<unsigned*>(g.d[1]);
-        unsigned* iy = ix + n;
-        if ((st = h2d(g.d[0], lambda, n * sizeof(double), s)) != RTB_OK) return st;
-        if ((st = h2d(ix, ccd_X, n * sizeof(unsigned), s)) != RTB_OK) return st;
-        if ((st = h2d(iy, ccd_Y, n * sizeof(unsigned), s)) != RTB_OK) return st;
+        g.add(lambda, n * sizeof(double), true, false);
+        g.add(ccd_X, n * sizeof(unsigned), true, false);
+        g.add(ccd_Y, n * sizeof(unsigned), true, false);
+    }
+    if ((st = g.open(true)) != RTB_OK) return st;
+    if (n) {
         double pix_area = xpix * ypix * 1.0E-2;  // ccd.cu:360
-        k_ccd_image<<<grid_for(n, 256, 8), 256, 0, s>>>(n, ix, iy, g.d[0], kb.as<double>(), qo, qn, so, sn, xdim, ydim,
-                                                          pix_area, img.as<double>(), g.counter, g.err);
+        k_ccd_image<<<g.grid(n), 256, 0, s>>>(n, g.as<unsigned>(2), g.as<unsigned>(3), g.d(1), g.d(0), qo, qn,
+                                                          so, sn, xdim, ydim, pix_area, img.as<double>(), g.counter,
+                                                          g.err);
     }
     if ((st = d2h(image, img.p, npix * sizeof(double), s)) != RTB_OK) return st;
     size_t outside = 0;
-    st = finish(s, g.err, &outside, g.counter);
+    st = g.close(&outside);
     if (st == RTB_OK && n_outside) *n_outside += outside;
     return st;
 }
@@ -914,14 +973,13 @@ extern "C" int rtb_grating_energy_distr(size_t n, const double* lambda, long ord
     int st = ensure_init();
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
-    Staged g;
-    if ((st = g.init(n, 2, false, s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[0], lambda, n * sizeof(double), s)) != RTB_OK) return st;
-    if ((st = h2d(g.d[1], energy_distr, n * sizeof(double), s)) != RTB_OK) return st;
-    k_grating_energy<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d[0], (long long)order, blaze_angle, alpha, gamma,
-                                                          gr_const, rule_start, rule_stop, g.d[1]);
-    if ((st = d2h(energy_distr, g.d[1], n * sizeof(double), s)) != RTB_OK) return st;
-    return finish(s, nullptr, nullptr, nullptr);
+    HostArrays g(s);
+    g.add(lambda, n * sizeof(double), true, false);
+    g.add(energy_distr, n * sizeof(double), true, true);
+    if ((st = g.open(false)) != RTB_OK) return st;
+    k_grating_energy<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d(0), (long long)order, blaze_angle, alpha, gamma,
+                                                          gr_const, rule_start, rule_stop, g.d(1));
+    return g.close();
 }
 
 extern "C" int rtb_qe_curves(const rtb_qe_surface* surfaces, size_t n_surfaces, const double* rows, size_t n_rows,
@@ -986,5 +1044,5 @@ extern "C" int rtb_qe_curves(const rtb_qe_surface* surfaces, size_t n_surfaces, 
                                                           from_rows, d_l, d_q, err);
     if ((st = d2h(lambda, d_l, b_out, s)) != RTB_OK) return st;
     if ((st = d2h(qe, d_q, b_out, s)) != RTB_OK) return st;
-    return finish(s, err, nullptr, nullptr);
+    return finish(s, err);
 }

@@ -110,6 +110,10 @@ struct DevBuf {
     }
 };
 
+// Whether [p, p + bytes) lies within a page-locked vector of the library's
+// (rtb_alocate_vector), which the device can read and write in place.
+bool in_host_vector(const void* p, size_t bytes);
+
 // ---- trace plumbing shared by the C ABI files (trace.cu) ----
 
 struct Lock {

@@ -131,7 +131,7 @@ __global__ void k_fused_mixed(const DevScheme* sch, const double* knots, const D
 // ---- ordering (order.cu) ----
 int reference_order(const DevBeam* h_beams, int n_beams, int n_stages, const DevRays& rays, uint32_t* order,
                     cudaStream_t stream);
-int rearrange_device(size_t n_good, double* arrays[7], char* flag, size_t* n_good_out, cudaStream_t stream);
+int rearrange_host(size_t n_good, double* const arrays[7], char* flag, size_t* n_good_out, cudaStream_t stream);
 
 #endif
 

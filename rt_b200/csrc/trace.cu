@@ -320,25 +320,8 @@ int rtb_rearrange(size_t* n_good, double* X, double* Y, double* Z, double* cX, d
     Lock l;
     int st = ensure_init();
     if (st != RTB_OK) return st;
-    cudaStream_t s = engine().stream;
-    DevBuf buf;
-    if ((st = buf.alloc(ng * (7 * sizeof(double) + 1), s)) != RTB_OK) return st;
     double* host[7] = {X, Y, Z, cX, cY, cZ, lambda};
-    double* dev[7];
-    for (int i = 0; i < 7; ++i) {
-        dev[i] = buf.as<double>() + (size_t)i * ng;
-        RTB_CUDA_TRY(cudaMemcpyAsync(dev[i], host[i], ng * sizeof(double), cudaMemcpyHostToDevice, s));
-    }
-    char* dflag = reinterpret_cast<char*>(buf.as<double>() + 7 * ng);
-    RTB_CUDA_TRY(cudaMemcpyAsync(dflag, flag, ng, cudaMemcpyHostToDevice, s));
-    size_t ng_out = ng;
-    if ((st = rearrange_device(ng, dev, dflag, &ng_out, s)) != RTB_OK) return st;
-    for (int i = 0; i < 7; ++i)
-        RTB_CUDA_TRY(cudaMemcpyAsync(host[i], dev[i], ng * sizeof(double), cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaMemcpyAsync(flag, dflag, ng, cudaMemcpyDeviceToHost, s));
-    RTB_CUDA_TRY(cudaStreamSynchronize(s));
-    *n_good = ng_out;
-    return RTB_OK;
+    return rearrange_host(ng, host, flag, n_good, engine().stream);
 }
 
 }  // extern "C"
