@@ -18,6 +18,7 @@ struct Engine {
     int sm_count = 148;
     int max_smem_optin = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t copy_streams[2] = {nullptr, nullptr};  // rtb_trace_host's, made at its first call
 };
 
 Engine& engine();
@@ -209,7 +210,8 @@ FrameArgs frame_args(const rtb_trace_opts* o);
 // out_by_slot: outputs at the tracing slot instead of the ray's index.
 int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_trace_opts& o, const DevRays& in,
                  const DevRays& out, const FrameArgs& frame, cudaStream_t st, const uint32_t* order = nullptr,
-                 bool in_by_slot = false, const void* rows = nullptr, bool out_by_slot = false);
+                 bool in_by_slot = false, const void* rows = nullptr, bool out_by_slot = false,
+                 unsigned max_blocks = 0);
 // The coherent tracing order (beam, chunk, wavelength, Morton code of the
 // entrance position) of n <= 2^32 generated rays, as a permutation in
 // `order` (device, n).

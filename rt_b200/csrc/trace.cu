@@ -124,7 +124,7 @@ int default_rpt(int precision, uint64_t n_rays) {
 
 int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_trace_opts& o, const DevRays& in,
                  const DevRays& out, const FrameArgs& frame, cudaStream_t st, const uint32_t* order,
-                 bool in_by_slot, const void* rows, bool out_by_slot) {
+                 bool in_by_slot, const void* rows, bool out_by_slot, unsigned max_blocks) {
     if (o.engine == RTB_ENGINE_PER_SURFACE) {
         if (o.precision != RTB_FP64) return RTB_BAD_VALUE;
         unsigned grid = grid_for(in.n, 256, 8);
@@ -158,6 +158,7 @@ int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_
         RTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
         if (per_sm < 1) per_sm = 1;
         unsigned grid = grid_for(in.n, threads * rpt, per_sm);
+        if (max_blocks && grid > max_blocks) grid = max_blocks;
         // the fused kernels' parameters, in order
         const DevScheme* sch = a.sch;
         const double* knots = a.knots;
@@ -328,7 +329,40 @@ int rtb_rearrange(size_t* n_good, double* X, double* Y, double* Z, double* cX, d
 
 namespace rtb {
 
-// rtb_trace over host arrays: chunks of rays cycle through two device
+// Whether rtb_trace_host traces the arrays where they lie: all of them library
+// vectors (rtb_alocate_vector) apart from one another, the beams covering every
+// ray, and not so many rays that the copy engines' higher rate pays for the
+// first chunk's copy-in and the last one's copy-out, when only one direction
+// of the link is busy (kHostInPlace).
+constexpr uint64_t kHostInPlace = 1ull << 24;
+static bool host_in_place(const rtb_rays* h, const std::vector<DevBeam>& db) {
+    const uint64_t n = h->n;
+    if (n > kHostInPlace || !h->lost_stage) return false;
+    uint64_t covered = 0;
+    for (const DevBeam& b : db) covered += b.n_rays;
+    if (covered != n) return false;
+    const void* p[9] = {h->X, h->Y, h->Z, h->cX, h->cY, h->cZ, h->lambda, h->flag, h->lost_stage};
+    for (int i = 0; i < 9; ++i) {
+        const size_t bytes = i < 7 ? n * sizeof(double) : n;
+        if (!in_host_vector(p[i], bytes)) return false;
+        for (int j = 0; j < i; ++j) {
+            const char *a = static_cast<const char*>(p[i]), *b = static_cast<const char*>(p[j]);
+            if (a < b + (j < 7 ? n * sizeof(double) : n) && b < a + bytes) return false;
+        }
+    }
+    return true;
+}
+
+// rtb_trace over host arrays.  Library vectors are traced in place: the fused
+// kernel loads the rays over the link and stores its results there, both
+// directions busy from its second row on, with one block per SM (more of them
+// put all their loads before the first stores, fewer do not keep the link
+// busy).  C1, us in place at 64 / 148 / 592 blocks and in the chunks below:
+// mixed 1e5 rays 340 / 305 / 351, 469; 1e6 1530 / 1380 / 1543, 2035; 4e6 5099 /
+// 4926 / 5373, 5756; FP64 1e6 2074 / 1343 / 1396, 1960.  The link's 57 bytes a
+// ray at 46 GB/s, where the copy engines reach 50 (1e8 rays).
+//
+// Other arrays and more rays: chunks of rays cycle through two device
 // buffers on two streams, so that the copy-in of one chunk, the trace of the
 // previous one and the copy-out of the one before overlap.  Page-locked host
 // arrays (rtb_alocate_vector) are needed for the copies to be asynchronous.
@@ -342,12 +376,33 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
     if ((st = check_beams(beams, n_beams, h->n, db, &ps.sch)) != RTB_OK) return st;
     const uint64_t n = h->n;
     if (n == 0) return RTB_OK;
+    rtb_trace_opts o = *opts;
+    o.engine = RTB_ENGINE_FUSED;
+    int dev = -1;
+    RTB_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev == engine().device && host_in_place(h, db)) {
+        cudaStream_t s = engine().stream;
+        TraceArgs a;
+        if ((st = a.init(ps, db, s)) != RTB_OK) return st;
+        const DevRays rays = dev_rays(h);
+        if ((st = launch_trace(ps, a, (int)n_beams, o, rays, rays, frame_args(opts), s, nullptr, false, nullptr, false,
+                               (unsigned)engine().sm_count)) != RTB_OK)
+            return st;
+        std::vector<unsigned long long> counts(a.counts_len + 1);
+        if ((st = a.fetch(counts.data(), s)) != RTB_OK) return st;
+        RTB_CUDA_TRY(cudaStreamSynchronize(s));
+        return trace_result(ps, counts.data(), (unsigned)counts[a.counts_len], (int)n_beams, stats);
+    }
     if (chunk == 0) chunk = (size_t)1 << 22;
     if (chunk > n) chunk = n;
     const size_t per_ray = 7 * sizeof(double) + 2;
     const int ns1 = 3 * ps.sch.n_surfaces + 1;
-    cudaStream_t streams[2] = {nullptr, nullptr};
-    for (auto& s : streams) RTB_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    // the streams are kept (making and ending two took 0.3 ms), except on a
+    // device other than the library's
+    cudaStream_t own[2] = {nullptr, nullptr};
+    cudaStream_t* streams = dev == engine().device ? engine().copy_streams : own;
+    for (int i = 0; i < 2; ++i)
+        if (!streams[i]) RTB_CUDA_TRY(cudaStreamCreateWithFlags(&streams[i], cudaStreamNonBlocking));
     // Per slot: device rays of one chunk, the trace arguments (scheme and
     // knots uploaded once), and page-locked staging for the chunk's beam
     // table and its counters.  Page-locked, so that no copy of a chunk blocks
@@ -404,8 +459,6 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
     std::vector<unsigned long long> total((size_t)n_beams * ns1, 0);
     unsigned err_all = 0;
     FrameArgs frame = frame_args(opts);
-    rtb_trace_opts o = *opts;
-    o.engine = RTB_ENGINE_FUSED;
     double* hin[7] = {h->X, h->Y, h->Z, h->cX, h->cY, h->cZ, h->lambda};
     auto drain = [&](Slot& sl, cudaStream_t s) -> int {
         RTB_CUDA_TRY(cudaStreamSynchronize(s));
@@ -487,10 +540,9 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
         slots[i].args.buf.release();
         slots[i].buf.release();
     }
-    for (auto& s : streams) {
-        if (!s) continue;
-        cudaStreamSynchronize(s);
-        cudaStreamDestroy(s);
+    for (int i = 0; i < 2; ++i) {
+        if (streams[i]) cudaStreamSynchronize(streams[i]);
+        if (own[i]) cudaStreamDestroy(own[i]);
     }
     if (h_stage) cudaFreeHost(h_stage);
     if (st != RTB_OK) return st;

@@ -125,3 +125,47 @@ def test_shared_arrays_are_read_as_they_were():
         assert np.array_equal(*results)
     finally:
         vec.free()
+
+
+class PlainRays:
+    """Ordinary host arrays with the fields rtb_trace_host takes."""
+
+    def __init__(self, n):
+        self.n = n
+        for f in E.FIELDS:
+            setattr(self, f, np.zeros(n))
+        self.flag, self.lost_stage = np.ones(n, np.int8), np.zeros(n, np.uint8)
+
+    def struct(self):
+        return ffi.Rays(*(ffi.vptr(getattr(self, f)) for f in E.FIELDS), ffi.vptr(self.flag),
+                        ffi.vptr(self.lost_stage), self.n)
+
+
+@pytest.mark.parametrize("n", [1, 4097, 65_536, 65_537, 700_001])
+@pytest.mark.parametrize("precision", [ffi.FP64, ffi.MIXED, ffi.MIXED32])
+@pytest.mark.parametrize("state_out", [0, 1])
+def test_host_trace_of_library_vectors(n, precision, state_out):
+    """Rays traced in place have the results of copied arrays; rays that are not
+    traced and survivors' lost stages stay as they were."""
+    surf = S.to_c(S.echelle(), E.spline_init).surfaces
+    k = n // 3
+    beams = [S.make_beam(0, k, 1, S.C1_RADIUS, (0.6, 0.6), 3, orders=(45, 1)),
+             S.make_beam(k, n - k, 1, S.C1_RADIUS, (0.62, 0.62), 4, orders=(46, 1))]
+    if k == 0:
+        beams = beams[1:]
+    source = E.generate(beams, n)
+    rng = np.random.default_rng(n)
+    flag, stage = (rng.random(n) < 0.95).astype(np.int8), rng.integers(0, 255, n).astype(np.uint8)
+    results = []
+    for rays in (PlainRays(n), E.PinnedRays(n)):
+        for f in E.FIELDS:
+            getattr(rays, f)[:] = getattr(source, f).cpu().numpy()
+        rays.flag[:], rays.lost_stage[:] = flag, stage
+        st, stats = E.trace_host(surf, beams, rays, E.opts(precision=precision, fixes=3, state_out=state_out))
+        results.append([st, stats.ray_surfaces, stats.n_good] +
+                       [getattr(rays, f).copy() for f in E.FIELDS + ("flag", "lost_stage")])
+    for a, b in zip(*results):
+        if isinstance(a, np.ndarray):
+            assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+        else:
+            assert a == b
