@@ -57,14 +57,17 @@ struct RtSurfacesF64 {
 
 // Fused FP64 trace: the whole surface sequence per ray in registers, the
 // scheme and knot tables in shared memory, a persistent grid whose blocks
-// take tiles of blockDim x rpt rays from the counter.  The block steps
-// through the surfaces together (a barrier after each): the bit-exact code of
-// all surface kinds is larger than the instruction cache, and warps spread
-// over different surfaces missed it on most issues (ncu: 12 cycles of
-// no_instruction stall per issued instruction, C1 29.8 ms); in step, one
-// surface's code serves the whole block (24.5 ms).  Bit-identical to
-// k_surface_step.  With a frame, good rays add their pixel with
-// warp-aggregated atomics.
+// take tiles of blockDim x rpt rays from the counter.  The block meets at
+// every tile and, in the kernel for any scheme, steps through the surfaces
+// together (a barrier after each): the bit-exact code of all surface kinds is
+// larger than the instruction cache, and warps spread over different surfaces
+// missed it on most issues (ncu: 12 cycles of no_instruction stall per issued
+// instruction, C1 29.8 ms); in step, one surface's code serves the whole block
+// (24.5 ms).  A kernel compiled for its scheme keeps together well enough by
+// meeting at each tile of one ray per thread (2e7 C1 rays 2.84 ms; 2.89 with a
+// barrier per surface, 3.40 with tiles per warp and no barrier at all).
+// Bit-identical to k_surface_step.  With a frame, good rays add their pixel
+// with warp-aggregated atomics.
 template <class Surfaces>
 __device__ __forceinline__ void fused_fp64(const DevScheme* __restrict__ g_sch, const double* knots,
                                            const DevBeam* beams, int n_beams, DevRays in, DevRays out,

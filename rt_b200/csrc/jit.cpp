@@ -246,7 +246,7 @@ std::string scheme_source(const DevScheme& sch, int precision) {
         for (int k = 0; k < sch.n_surfaces; ++k) {
             const std::string ks = std::to_string(k);
             src += "        if (stage == -1) f64_surface<" + fixed_shape(sch.s[k]) + ">(" + S + ks + "], " + ks + ", " +
-                   F + ", knots, beams, b, lam, err, r, stage);\n        __syncthreads();\n";
+                   F + ", knots, beams, b, lam, err, r, stage);\n";
         }
         src += std::string("    }\n};\n}  // namespace rtb\n"
                            "extern \"C\" __global__ void __maxnreg__(" + maxnreg + ") ") + kFp64Name + "(\n" + kParams +
