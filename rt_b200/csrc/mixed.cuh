@@ -602,6 +602,7 @@ __device__ __forceinline__ void fused_mixed(const DevScheme* __restrict__ g_sch,
     RowLoop rows(ts, in.n, warp_row_buffer<Row64>(ts.n_surfaces, ts.n_knots), (unsigned)sizeof(Row64), err);
     const int lane = threadIdx.x & 31;
     BeamCursor cur;
+    EventCounter events;
     while (rows.begin()) {
         const size_t slot = rows.slot();
         const bool valid = slot < in.n;
@@ -667,9 +668,11 @@ __device__ __forceinline__ void fused_mixed(const DevScheme* __restrict__ g_sch,
         } else if (valid && (rows.packed || in.flag != out.flag)) {
             out.flag[oi] = f;
         }
-        count_event(ev, key, counts);
+        events.add(ev, key, counts);
+        if (ts.rpt == 1) events.flush(counts);  // a small trace: not all warps' at the end
         if (frame.counts) frame_add<false>(good, outX, outY, frame);
     }
+    events.flush(counts);
 }
 
 }  // namespace rtb

@@ -92,6 +92,39 @@ __device__ __forceinline__ void count_event(bool ev, int key, unsigned long long
     if ((threadIdx.x & 31) == (unsigned)(__ffs(same) - 1)) atomicAdd(counts + key, (unsigned long long)__popc(same));
 }
 
+// The same for the persistent kernels, whose warps see one counter many times
+// in a row (the rays of a row mostly share a beam and a fate): the warp keeps
+// the sum of one counter and adds it when the counter changes and at the end.
+// Every lane of the warp calls add and flush.  One atomic per warp and row on
+// a single address bound schemes of few surfaces: C0 mixed, 6e6 rays in one
+// beam 0.216 -> 0.148 ms; C1, 1e8 rays in 31 beams 3.86 -> 3.72.  The FP64
+// kernel, slower per row, gains nothing (1 % slower) and counts row by row.
+struct EventCounter {
+    int key = -1;
+    unsigned n = 0;
+    __device__ __forceinline__ void add(bool ev, int k, unsigned long long* counts) {
+        const unsigned events = __ballot_sync(0xffffffffu, ev);
+        unsigned other = __ballot_sync(0xffffffffu, ev && k != key);
+        if (other) {
+            if (other == events) {  // none of them the counter kept: keep the first one's
+                flush(counts);
+                key = __shfl_sync(0xffffffffu, k, __ffs(events) - 1);
+                other = __ballot_sync(0xffffffffu, ev && k != key);
+            }
+            if (ev && k != key) {
+                const unsigned same = __match_any_sync(other, k);
+                if ((threadIdx.x & 31) == (unsigned)(__ffs(same) - 1))
+                    atomicAdd(counts + k, (unsigned long long)__popc(same));
+            }
+        }
+        n += (unsigned)__popc(events & ~other);
+    }
+    __device__ __forceinline__ void flush(unsigned long long* counts) {
+        if (n && (threadIdx.x & 31) == 0) atomicAdd(counts + key, (unsigned long long)n);
+        n = 0;
+    }
+};
+
 // Frame counts of one good ray at the detector: warp-aggregated increments
 // of the pixel it lands on.  Non-finite coordinates count as outside.  The
 // FP64 kernels divide by the pixel size as the reference does; the mixed
