@@ -430,7 +430,7 @@ RTB_API int rtb_plan_specialized(const rtb_plan* plan, int32_t* specialized, cha
  * to this scheme's structure ahead of rtb_plan_create (which compiles it
  * otherwise, once per structure and process); needs no device.  Once
  * compiled, one-shot fused traces of that precision and a scheme of that
- * structure (rtb_trace, rtb_trace_out, rtb_trace_host) launch it too; they
+ * structure (rtb_trace, rtb_trace_out, an FP64 rtb_trace_host) launch it too; they
  * never compile it themselves.  RTB_OK when compiled; RTB_FAILED with the
  * reason in note (may be NULL) when NVRTC is unavailable or fails.  With
  * RTB_JIT_CACHE=<directory> in the environment, compiled kernels are also

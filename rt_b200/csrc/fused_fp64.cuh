@@ -91,9 +91,6 @@ __device__ __forceinline__ void fused_fp64(const DevScheme* __restrict__ g_sch, 
             const size_t i = (ts.order && slot < in.n) ? (size_t)ts.order[slot] : slot;
             const size_t ri = ts.in_by_slot ? slot : i;
             const size_t oi = ts.out_by_slot ? slot : i;  // where its results go
-            bool ev = false, good = false;
-            int key = 0;
-            double outX = 0, outY = 0;
             const bool have = slot < in.n && in.flag[ri] == 1;
             f64::Ray r{0, 0, 0, 0, 0, 0};
             double lam = 0;
@@ -107,36 +104,28 @@ __device__ __forceinline__ void fused_fp64(const DevScheme* __restrict__ g_sch, 
             }
             int stage = have ? -1 : -3;
             Surfaces::run(sch, s_knots, beams, b, lam, err, r, stage);
-            if (have) {
-                if (stage >= 0) {
-                    ev = true;
-                    if (sch->renorm_lost) f64::renormalize(r, Surfaces::renorm_after(sch, stage / 3));
-                    out.flag[oi] = 0;
-                    out.lost_stage[oi] = (uint8_t)stage;
-                    key = b * (n_stages + 1) + stage;
-                } else if (stage == -1) {
-                    ev = good = true;
-                    key = b * (n_stages + 1) + n_stages;
-                    if (in.flag != out.flag) {
-                        out.flag[oi] = 1;
-                        out.lost_stage[oi] = RTB_NOT_LOST;
-                    }
+            if (stage >= 0 && sch->renorm_lost) f64::renormalize(r, Surfaces::renorm_after(sch, stage / 3));
+            const bool ev = stage >= -1, good = stage == -1;  // -2: the kernel's error; -3: no ray
+            // the lanes store together: whole lines over the link (C1 compiled for
+            // the scheme, 1e6 rays in place 3347 -> 1588 us, 1e7 device rays 2.97 -> 2.87 ms)
+            __syncwarp();
+            if (ev) {
+                if (!good || in.flag != out.flag) {
+                    out.flag[oi] = good;
+                    out.lost_stage[oi] = good ? RTB_NOT_LOST : (uint8_t)stage;
                 }
-                if (stage != -2) {
-                    out.X[oi] = r.X;
-                    out.Y[oi] = r.Y;
-                    if (state_out) {
-                        out.Z[oi] = r.Z;
-                        out.cX[oi] = r.cX;
-                        out.cY[oi] = r.cY;
-                        out.cZ[oi] = r.cZ;
-                    }
+                out.X[oi] = r.X;
+                out.Y[oi] = r.Y;
+                if (state_out) {
+                    out.Z[oi] = r.Z;
+                    out.cX[oi] = r.cX;
+                    out.cY[oi] = r.cY;
+                    out.cZ[oi] = r.cZ;
                 }
-                outX = r.X;
-                outY = r.Y;
             }
+            const int key = b * (n_stages + 1) + (good ? n_stages : stage);
             count_event(ev, key, counts);
-            if (frame.counts) frame_add(good, outX, outY, frame);
+            if (frame.counts) frame_add(good, r.X, r.Y, frame);
         }
     }
 }

@@ -361,6 +361,11 @@ static bool host_in_place(const rtb_rays* h, const std::vector<DevBeam>& db) {
 // mixed 1e5 rays 340 / 305 / 351, 469; 1e6 1530 / 1380 / 1543, 2035; 4e6 5099 /
 // 4926 / 5373, 5756; FP64 1e6 2074 / 1343 / 1396, 1960.  The link's 57 bytes a
 // ray at 46 GB/s, where the copy engines reach 50 (1e8 rays).
+// The mixed kernels compiled for a scheme are left to device arrays: their
+// lanes come to the stores in groups, which the link carries as partial lines
+// (C1, 1e6 rays, X and Y back 2573 us, all of the state back 4280; the kernels
+// for any scheme 1362 and 1680).  Meeting before the stores cures it too but
+// costs plans 1.2 %, and the link is the bound with either kernel.
 //
 // Other arrays and more rays: chunks of rays cycle through two device
 // buffers on two streams, so that the copy-in of one chunk, the trace of the
@@ -370,7 +375,7 @@ int trace_host_impl(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
                     const rtb_trace_opts* opts, const rtb_rays* h, rtb_trace_stats* stats, size_t chunk) {
     PreparedScheme ps;
     int st = prepare_scheme(surfaces, n_surfaces, opts->fixes, opts->renormalize_lost, opts->precision, ps);
-    if (st == RTB_OK) st = attach_compiled(ps, *opts);
+    if (st == RTB_OK && opts->precision == RTB_FP64) st = attach_compiled(ps, *opts);
     if (st != RTB_OK) return st;
     std::vector<DevBeam> db;
     if ((st = check_beams(beams, n_beams, h->n, db, &ps.sch)) != RTB_OK) return st;

@@ -169,3 +169,26 @@ def test_host_trace_of_library_vectors(n, precision, state_out):
             assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
         else:
             assert a == b
+
+
+@pytest.mark.parametrize("precision", [ffi.FP64, ffi.MIXED, ffi.MIXED32])
+@pytest.mark.parametrize("n", [33, 40_001])
+def test_host_trace_is_the_same_after_a_plan_of_its_scheme(n, precision):
+    """A plan compiles its scheme's kernel, which later calls of the scheme may take."""
+    surf = S.to_c(S.echelle(), E.spline_init).surfaces
+    beams = [S.make_beam(0, n, 1, S.C1_RADIUS, (0.61, 0.61), 5, orders=(45, 1))]
+    source = E.generate(beams, n)
+    o = E.opts(precision=precision, fixes=3, state_out=1)
+    results = []
+    for plan_first in (False, True):
+        if plan_first:
+            plan = E.Plan(surf, beams, o)
+        rays = E.PinnedRays(n)
+        for f in E.FIELDS + ("flag", "lost_stage"):
+            getattr(rays, f)[:] = getattr(source, f).cpu().numpy()
+        st, stats = E.trace_host(surf, beams, rays, o)
+        results.append([np.array([st, stats.ray_surfaces, stats.n_good])] +
+                       [getattr(rays, f).copy() for f in E.FIELDS + ("flag", "lost_stage")])
+    del plan
+    for a, b in zip(*results):
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
