@@ -327,7 +327,8 @@ RTB_API int rtb_trace_out_noalloc(const rtb_surface* surfaces, size_t n_surfaces
                                   size_t n_beams, const rtb_trace_opts* opts, const rtb_rays* in,
                                   const rtb_rays* out, rtb_trace_stats* stats, void* stream);
 
-/* rtb_trace on host arrays: copies in, traces and copies out, overlapping the
+/* rtb_trace on host arrays: traces library vectors (rtb_alocate_vector) of up
+ * to 2^24 rays where they lie; copies others in and out, overlapping the
  * copies of one chunk with the trace of another.  Synchronous. */
 RTB_API int rtb_trace_host(const rtb_surface* surfaces, size_t n_surfaces, const rtb_beam* beams,
                    size_t n_beams, const rtb_trace_opts* opts, const rtb_rays* host_rays,
