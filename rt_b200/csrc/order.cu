@@ -414,8 +414,10 @@ int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out,
     uint64_t lost = 0;
     RTB_CUDA_TRY(cudaMemcpyAsync(&lost, w.seg_lost, sizeof(lost), cudaMemcpyDeviceToHost, st));
     RTB_CUDA_TRY(cudaStreamSynchronize(st));
-    *ng_out = ng - lost;
-    if (lost == 0) return RTB_OK;
+    if (lost == 0) {
+        *ng_out = ng;
+        return RTB_OK;
+    }
     Arr7 arr;
     const bool in_place = lost <= ng / kSwapInPlace;
     for (int i = 0; i < 7; ++i) {
@@ -437,6 +439,7 @@ int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out,
             RTB_CUDA_TRY(cudaMemcpyAsync(host[i], arr.a[i], ng * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (dflag != flag) RTB_CUDA_TRY(cudaMemcpyAsync(flag, dflag, ng, cudaMemcpyDeviceToHost, st));
     RTB_CUDA_TRY(cudaStreamSynchronize(st));
+    *ng_out = ng - lost;  // only now: a call that fails leaves the caller's count with its rays
     return RTB_OK;
 }
 
