@@ -457,8 +457,9 @@ static void spline_second_derivatives(size_t N, const double* x, const double* y
 static std::mutex g_vectors_mu;
 static std::map<uintptr_t, size_t> g_vectors;
 
-bool in_host_vector(const void* p, size_t bytes) {
+bool in_host_vector(const void* p, size_t bytes, size_t align) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    if (at % align != 0) return false;
     std::lock_guard<std::mutex> g(g_vectors_mu);
     auto it = g_vectors.upper_bound(at);
     if (it == g_vectors.begin()) return false;
@@ -490,9 +491,12 @@ struct HostArrays {
     unsigned* err = nullptr;
     cudaStream_t st;
     explicit HostArrays(cudaStream_t s) : st(s) {}
-    void add(const void* host, size_t bytes, bool in, bool out) {
-        const bool staged = !in_host_vector(host, bytes);
-        e[n++] = Entry{const_cast<void*>(host), staged ? nullptr : const_cast<void*>(host), bytes, in, out, staged};
+    template <class T>
+    void add(const T* host, size_t count, bool in, bool out) {
+        const size_t bytes = count * sizeof(T);
+        const bool staged = !in_host_vector(host, bytes, sizeof(T));
+        void* p = const_cast<T*>(host);
+        e[n++] = Entry{p, staged ? nullptr : p, bytes, in, out, staged};
     }
     int open(bool counted) {
         // arrays that share memory are copied, so that each is read as it was
@@ -650,7 +654,7 @@ int rtb_beam_random(int shape, const double* params, const double* center, size_
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), false, true);
+    for (double* p : {X, Y, Z}) g.add(p, n, false, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_beam_random<<<g.grid(n), 256, 0, s>>>(n, params[1], params[2], center[0], center[1], center[2], seed,
                                                         first_ray, g.d(0), g.d(1), g.d(2));
@@ -717,7 +721,7 @@ int rtb_uniform_range_beam(size_t n, const double* range, double* lambda) {
     cudaStream_t s = engine().stream;
     double d_l = (range[1] - range[0]) / (n - 1);  // rt_cuda_engine_beam.cu:726
     HostArrays g(s);
-    g.add(lambda, n * sizeof(double), false, true);
+    g.add(lambda, n, false, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_uniform_range<<<g.grid(n), 256, 0, s>>>(n, range[0], d_l, g.d(0));
     return g.close();
@@ -731,7 +735,7 @@ int rtb_random_range_beam(size_t n, const double* range, double* lambda, uint64_
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    g.add(lambda, n * sizeof(double), false, true);
+    g.add(lambda, n, false, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_random_range<<<g.grid(n), 256, 0, s>>>(n, range[0], range[1], seed, g.d(0));
     return g.close();
@@ -749,7 +753,7 @@ int rtb_beam_transform(size_t n, const double* angles, const double* dist, doubl
     std::memset(&ds, 0, sizeof(ds));
     transform_constants(angles, dist, ds);
     HostArrays g(s);
-    for (double* p : {X, Y, Z, cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    for (double* p : {X, Y, Z, cX, cY, cZ}) g.add(p, n, true, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_transform<<<g.grid(n), 256, 0, s>>>(n, ds, g.d(0), g.d(1), g.d(2), g.d(3), g.d(4), g.d(5));
     return g.close();
@@ -766,8 +770,8 @@ static int intersection_impl(int cls, const double* params, size_t n, double* X,
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), true, true);
-    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, false);
+    for (double* p : {X, Y, Z}) g.add(p, n, true, true);
+    for (double* p : {cX, cY, cZ}) g.add(p, n, true, false);
     g.add(flag, n, true, true);
     if ((st = g.open(true)) != RTB_OK) return st;
     k_intersect<<<g.grid(n), 256, 0, s>>>(n, ds, fixes, g.d(0), g.d(1), g.d(2), g.d(3), g.d(4), g.d(5),
@@ -795,8 +799,8 @@ int rtb_surface_reflection(int cls, const double* params, size_t n, double* X, d
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), true, false);
-    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    for (double* p : {X, Y, Z}) g.add(p, n, true, false);
+    for (double* p : {cX, cY, cZ}) g.add(p, n, true, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_reflect<<<g.grid(n), 256, 0, s>>>(n, ds, g.d(0), g.d(1), g.d(2), g.d(3), g.d(4), g.d(5));
     return g.close();
@@ -823,11 +827,11 @@ static int action_impl(int type, int cls, int gr_type, const double* params, lon
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    for (double* p : {X, Y, Z}) g.add(p, n * sizeof(double), true, false);
-    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
-    g.add(lambda, n * sizeof(double), true, false);
+    for (double* p : {X, Y, Z}) g.add(p, n, true, false);
+    for (double* p : {cX, cY, cZ}) g.add(p, n, true, true);
+    g.add(lambda, n, true, false);
     g.add(flag, n, true, true);
-    g.add(knots.data(), knots.size() * sizeof(double), true, false);
+    g.add(knots.data(), knots.size(), true, false);
     if ((st = g.open(true)) != RTB_OK) return st;
     k_action<<<g.grid(n), 256, 0, s>>>(n, ds, g.d(8), (long long)order, g.d(6), g.d(0), g.d(1), g.d(2), g.d(3),
                                                    g.d(4), g.d(5), g.as<char>(7), g.counter, g.err);
@@ -859,9 +863,9 @@ int rtb_surface_QE(size_t n, const double* lambda, double* spec, const rtb_table
     if ((st = ensure_init()) != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    g.add(lambda, n * sizeof(double), true, false);
-    g.add(spec, n * sizeof(double), true, true);
-    g.add(knots.data(), knots.size() * sizeof(double), true, false);
+    g.add(lambda, n, true, false);
+    g.add(spec, n, true, true);
+    g.add(knots.data(), knots.size(), true, false);
     if ((st = g.open(true)) != RTB_OK) return st;
     k_surface_qe<<<g.grid(n), 256, 0, s>>>(n, g.d(0), g.d(1), g.d(2), off, cnt, g.err);
     return g.close();
@@ -874,7 +878,7 @@ int rtb_normalize(size_t n, double* cX, double* cY, double* cZ) {
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    for (double* p : {cX, cY, cZ}) g.add(p, n * sizeof(double), true, true);
+    for (double* p : {cX, cY, cZ}) g.add(p, n, true, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_normalize<<<g.grid(n), 256, 0, s>>>(n, g.d(0), g.d(1), g.d(2));
     return g.close();
@@ -890,8 +894,8 @@ int rtb_apply_constrains(int shade, int shape, const double* size, const double*
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    g.add(X, n * sizeof(double), true, false);
-    g.add(Y, n * sizeof(double), true, false);
+    g.add(X, n, true, false);
+    g.add(Y, n, true, false);
     g.add(flag, n, true, true);
     if ((st = g.open(true)) != RTB_OK) return st;
     k_aperture<<<g.grid(n), 256, 0, s>>>(n, shade, shape, size[0], shape == RTB_RECTANGLE ? size[1] : 0.0,
@@ -907,10 +911,10 @@ int rtb_ccd_coordinates(size_t n, const double* X, const double* Y, double xsize
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    g.add(X, n * sizeof(double), true, false);
-    g.add(Y, n * sizeof(double), true, false);
-    g.add(ccd_X, n * sizeof(unsigned), false, true);
-    g.add(ccd_Y, n * sizeof(unsigned), false, true);
+    g.add(X, n, true, false);
+    g.add(Y, n, true, false);
+    g.add(ccd_X, n, false, true);
+    g.add(ccd_Y, n, false, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_ccd_coords<<<g.grid(n), 256, 0, s>>>(n, g.d(0), g.d(1), xsize, ysize, xpix, ypix, g.as<unsigned>(2),
                                                        g.as<unsigned>(3));
@@ -937,11 +941,11 @@ int rtb_compute_ccd_image(size_t n, const unsigned int* ccd_X, const unsigned in
     if ((st = img.alloc(npix * sizeof(double), s)) != RTB_OK) return st;
     if ((st = h2d(img.p, image, npix * sizeof(double), s)) != RTB_OK) return st;
     HostArrays g(s);
-    g.add(knots.data(), knots.size() * sizeof(double), true, false);
+    g.add(knots.data(), knots.size(), true, false);
     if (n) {
-        g.add(lambda, n * sizeof(double), true, false);
-        g.add(ccd_X, n * sizeof(unsigned), true, false);
-        g.add(ccd_Y, n * sizeof(unsigned), true, false);
+        g.add(lambda, n, true, false);
+        g.add(ccd_X, n, true, false);
+        g.add(ccd_Y, n, true, false);
     }
     if ((st = g.open(true)) != RTB_OK) return st;
     if (n) {
@@ -974,8 +978,8 @@ extern "C" int rtb_grating_energy_distr(size_t n, const double* lambda, long ord
     if (st != RTB_OK) return st;
     cudaStream_t s = engine().stream;
     HostArrays g(s);
-    g.add(lambda, n * sizeof(double), true, false);
-    g.add(energy_distr, n * sizeof(double), true, true);
+    g.add(lambda, n, true, false);
+    g.add(energy_distr, n, true, true);
     if ((st = g.open(false)) != RTB_OK) return st;
     k_grating_energy<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d(0), (long long)order, blaze_angle, alpha, gamma,
                                                           gr_const, rule_start, rule_stop, g.d(1));

@@ -111,9 +111,11 @@ struct DevBuf {
     }
 };
 
-// Whether [p, p + bytes) lies within a page-locked vector of the library's
-// (rtb_alocate_vector), which the device can read and write in place.
-bool in_host_vector(const void* p, size_t bytes);
+// Whether the device can read and write [p, p + bytes) in place: it lies
+// within a page-locked vector of the library's (rtb_alocate_vector), at a
+// multiple of `align`, its elements' size (a kernel's load or store faults
+// where a copy takes any address).
+bool in_host_vector(const void* p, size_t bytes, size_t align);
 
 // ---- trace plumbing shared by the C ABI files (trace.cu) ----
 

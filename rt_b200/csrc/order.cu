@@ -397,7 +397,7 @@ int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out,
     Work w;
     int s = w.init(ng, 1, st);
     if (s != RTB_OK) return s;
-    bool vectors = in_host_vector(flag, ng);
+    bool vectors = in_host_vector(flag, ng, 1);
     char* dflag = flag;
     DevBuf fbuf, buf;
     if (!vectors) {
@@ -421,7 +421,7 @@ int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out,
     Arr7 arr;
     const bool in_place = lost <= ng / kSwapInPlace;
     for (int i = 0; i < 7; ++i) {
-        vectors = vectors && in_host_vector(host[i], ng * sizeof(double));
+        vectors = vectors && in_host_vector(host[i], ng * sizeof(double), sizeof(double));
         for (int j = 0; j < i; ++j)  // an array given twice is swapped once
             vectors = vectors && (host[i] + ng <= host[j] || host[j] + ng <= host[i]);
     }

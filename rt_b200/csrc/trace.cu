@@ -344,7 +344,7 @@ static bool host_in_place(const rtb_rays* h, const std::vector<DevBeam>& db) {
     const void* p[9] = {h->X, h->Y, h->Z, h->cX, h->cY, h->cZ, h->lambda, h->flag, h->lost_stage};
     for (int i = 0; i < 9; ++i) {
         const size_t bytes = i < 7 ? n * sizeof(double) : n;
-        if (!in_host_vector(p[i], bytes)) return false;
+        if (!in_host_vector(p[i], bytes, i < 7 ? sizeof(double) : 1)) return false;
         for (int j = 0; j < i; ++j) {
             const char *a = static_cast<const char*>(p[i]), *b = static_cast<const char*>(p[j]);
             if (a < b + (j < 7 ? n * sizeof(double) : n) && b < a + bytes) return false;
