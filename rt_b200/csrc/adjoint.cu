@@ -577,6 +577,20 @@ AdjArgs adj_args(const rtb_adjoint* c) {
     return a;
 }
 
+// Whether a kernel on `device` may store to the caller's array p: memory of
+// that device, elements aligned.  Any other (another device's, page-locked
+// host memory, an odd address) is left to a copy, which takes it or returns an
+// error where a store would fault.
+bool kernel_writes(const void* p, size_t align, int device) {
+    if (!p || reinterpret_cast<uintptr_t>(p) % align != 0) return false;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == device;
+}
+
 }  // namespace
 
 extern "C" {
@@ -734,9 +748,12 @@ int rtb_adjoint_forward(rtb_adjoint* c, const double* theta, const rtb_rays* ray
     RTB_CUDA_TRY(cudaMemcpyAsync(c->d_sch, h.data(), h.size(), cudaMemcpyHostToDevice, s));
     RTB_CUDA_TRY(cudaMemsetAsync(c->d_counts, 0, (nb * ns1 + 1) * 8, s));
     AdjArgs a = adj_args(c);
-    a.out_X = X;
-    a.out_Y = Y;
-    a.out_flag = flag;
+    // written by the kernel where it can store to them, copied otherwise
+    const bool to_X = kernel_writes(X, sizeof(double), c->device), to_Y = kernel_writes(Y, sizeof(double), c->device),
+               to_flag = kernel_writes(flag, 1, c->device);
+    a.out_X = to_X ? X : nullptr;
+    a.out_Y = to_Y ? Y : nullptr;
+    a.out_flag = to_flag ? flag : nullptr;
     DevRays in = dev_rays(rays);
     if (c->fwd_kernel) {
         unsigned long long* counts = c->d_counts;
@@ -748,6 +765,9 @@ int rtb_adjoint_forward(rtb_adjoint* c, const double* theta, const rtb_rays* ray
         k_adj_forward<<<adj_grid(c->n, kAdjForwardThreads), kAdjForwardThreads, 0, s>>>(a, in, c->d_counts, c->d_err);
     }
     RTB_CUDA_TRY(cudaGetLastError());
+    if (X && !to_X) RTB_CUDA_TRY(cudaMemcpyAsync(X, c->d_X, c->n * 8, cudaMemcpyDeviceToDevice, s));
+    if (Y && !to_Y) RTB_CUDA_TRY(cudaMemcpyAsync(Y, c->d_Y, c->n * 8, cudaMemcpyDeviceToDevice, s));
+    if (flag && !to_flag) RTB_CUDA_TRY(cudaMemcpyAsync(flag, c->d_flag, c->n, cudaMemcpyDeviceToDevice, s));
     std::vector<unsigned long long> counts(nb * ns1 + 1);  // and the error word
     RTB_CUDA_TRY(cudaMemcpyAsync(counts.data(), c->d_counts, counts.size() * 8, cudaMemcpyDeviceToHost, s));
     RTB_CUDA_TRY(cudaStreamSynchronize(s));
