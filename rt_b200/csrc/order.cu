@@ -8,9 +8,9 @@
 // is computed in parallel from a prefix sum of the lost marks.
 //
 // reference_order() replays the Rearrange calls of a whole trace from the
-// per-ray lost stages (one partition per stage with losses, all beams at
-// once, in one cooperative launch), giving the order in which the reference's
-// Beam::Save writes rays.
+// per-ray lost stages (one partition per stage with losses), giving the order
+// in which the reference's Beam::Save writes rays: beams of a few hundred rays
+// by a warp each, the others all at once in one cooperative launch.
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
@@ -138,6 +138,7 @@ namespace {
 // The replay of a whole trace's Rearrange calls (k_replay).  A segment (beam)
 // is cut into tiles of kTile positions; `stage` holds the lost stage of the
 // ray at each position, a tile's kTile bytes together, and follows the swaps.
+// Beams of up to kSmallSeg rays are replayed by k_replay_small.
 constexpr int kTile = 4096, kReplayThreads = 256, kPer = kTile / kReplayThreads;
 
 struct ReplaySeg {
@@ -151,7 +152,6 @@ struct Replay {
     ReplaySeg* segs;
     int n_segs, n_stages;
     uint32_t n_tiles;
-    uint64_t n;
     const uint8_t* lost_stage;
     uint32_t* order;         // beam-local index of the ray at each position
     uint8_t* stage;
@@ -162,7 +162,7 @@ struct Replay {
 
 __device__ __forceinline__ int seg_of_tile(const Replay& r, uint32_t t) {
     int lo = 0, hi = r.n_segs - 1;
-    while (lo < hi) {  // the last segment that starts at or before tile t: empty ones have no tiles
+    while (lo < hi) {  // the last segment that starts at or before tile t
         const int mid = (lo + hi + 1) >> 1;
         if (r.segs[mid].tile0 <= t) lo = mid; else hi = mid - 1;
     }
@@ -220,12 +220,6 @@ __global__ void __launch_bounds__(kReplayThreads, 4) k_replay(Replay r) {
         while (s + 1 < r.n_segs && r.segs[s + 1].tile0 <= t) ++s;
         return s;
     };
-    // positions outside every segment, relative to the segment before them
-    for (int g = (int)blockIdx.x - 1; g < r.n_segs; g += (int)gridDim.x) {
-        const uint64_t from = g < 0 ? 0 : r.segs[g].start + r.segs[g].n, base = r.segs[g < 0 ? 0 : g].start;
-        const uint64_t to = g + 1 < r.n_segs ? r.segs[g + 1].start : r.n;
-        for (uint64_t k = from + threadIdx.x; k < to; k += kReplayThreads) r.order[k] = (uint32_t)(k - base);
-    }
     unsigned seen[3] = {0, 0, 0};
     int s = first_seg;
     for (uint32_t t = t0; t < t1; ++t) {
@@ -340,6 +334,102 @@ __global__ void __launch_bounds__(kReplayThreads, 4) k_replay(Replay r) {
     }
 }
 
+// A beam of few rays, by one warp: its rays' stages and order in shared memory,
+// the stages that lost rays in turn, with the pairing of k_replay (ranks from
+// ballots, 32 positions at a time).  A tile of k_replay per beam would cost a
+// block three barriers a stage and kTile bytes of `stage` whatever the beam's
+// size: 1e5 beams of 10 rays took 11.3 ms and 410 MB so, 2.5 ms and 3 MB this
+// way, 1e4 of 100 rays 1.47 and 0.27 ms (the host's check of the beam table
+// with it).  The line lies where a tile's bytes come to 8 a ray, so that the
+// replay's scratch stays below 16 a ray; 1000 beams of 500 rays take 57 us here,
+// of 600 in k_replay 170.
+constexpr int kSmallSeg = 512, kSmallWarps = 8;
+
+struct SmallSeg {
+    uint64_t start;
+    uint32_t n, pad;
+};
+
+__global__ void __launch_bounds__(32 * kSmallWarps) k_replay_small(const SmallSeg* segs, int n_segs, int n_stages,
+                                                                   const uint8_t* lost_stage, uint32_t* order) {
+    __shared__ uint8_t s_stage[kSmallWarps][kSmallSeg];
+    __shared__ uint16_t s_order[kSmallWarps][kSmallSeg];
+    __shared__ uint16_t s_front[kSmallWarps][kSmallSeg / 2], s_back[kSmallWarps][kSmallSeg / 2];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    uint8_t* const stage = s_stage[warp];
+    uint16_t *const ord = s_order[warp], *const front = s_front[warp], *const back = s_back[warp];
+    for (int q = (int)(blockIdx.x * kSmallWarps + warp); q < n_segs; q += (int)(gridDim.x * kSmallWarps)) {
+        const uint64_t start = segs[q].start;
+        const int n = (int)segs[q].n;
+        unsigned seen[3] = {0, 0, 0};
+        for (int j = (int)lane; j < n; j += 32) {
+            const unsigned v = lost_stage[start + j];
+            stage[j] = (uint8_t)v;
+            ord[j] = (uint16_t)j;
+            if (v < (unsigned)n_stages) {
+                const unsigned bit = 1u << (v & 31);
+                if (v < 32) seen[0] |= bit;
+                else if (v < 64) seen[1] |= bit;
+                else seen[2] |= bit;
+            }
+        }
+        __syncwarp();
+        int ng = n;
+#pragma unroll
+        for (int w = 0; w < 3; ++w) {
+            for (unsigned left = __reduce_or_sync(0xffffffffu, seen[w]); left; left &= left - 1) {
+                const unsigned st = 32u * w + __ffs(left) - 1;
+                int lost = 0;
+                for (int j0 = 0; j0 < ng; j0 += 32) {
+                    const int j = j0 + (int)lane;
+                    lost += __popc(__ballot_sync(0xffffffffu, j < ng && stage[j] == st));
+                }
+                const int keep = ng - lost;
+                int pairs = 0, backs = 0;
+                for (int j0 = 0; j0 < keep; j0 += 32) {  // lost rays at the front
+                    const int j = j0 + (int)lane;
+                    const bool hit = j < keep && stage[j] == st;
+                    const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                    if (hit) front[pairs + __popc(hits & below)] = (uint16_t)j;
+                    pairs += __popc(hits);
+                }
+                for (int j0 = ng - 1; j0 >= keep; j0 -= 32) {  // good rays at the back, from the end
+                    const int j = j0 - (int)lane;
+                    const bool hit = j >= keep && stage[j] != st;
+                    const unsigned hits = __ballot_sync(0xffffffffu, hit);
+                    if (hit) back[backs + __popc(hits & below)] = (uint16_t)j;
+                    backs += __popc(hits);
+                }
+                __syncwarp();
+                for (int k = (int)lane; k < pairs; k += 32) {
+                    const int a = front[k], b = back[k];
+                    const uint16_t o = ord[a];
+                    ord[a] = ord[b];
+                    ord[b] = o;
+                    stage[a] = stage[b];  // position b leaves the good rays: its stage is not read again
+                }
+                __syncwarp();
+                ng = keep;
+            }
+        }
+        for (int j = (int)lane; j < n; j += 32) order[start + j] = ord[j];
+        __syncwarp();
+    }
+}
+
+// Positions outside every segment, relative to the segment before them (or the
+// first); the others are written after this.
+__global__ void k_iota(uint64_t n, const uint64_t* starts, int n_segs, uint32_t* order) {
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n; k += (uint64_t)blockDim.x * gridDim.x) {
+        int lo = 0, hi = n_segs - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (starts[mid] <= k) lo = mid; else hi = mid - 1;
+        }
+        order[k] = (uint32_t)(k - starts[lo]);
+    }
+}
+
 }  // namespace
 
 int reference_order(const DevBeam* h_beams, int n_beams, int n_stages, const DevRays& rays, uint32_t* order,
@@ -347,27 +437,54 @@ int reference_order(const DevBeam* h_beams, int n_beams, int n_stages, const Dev
     const uint64_t n = rays.n;
     if (n == 0) return RTB_OK;
     if (n > 0xFFFFFFFFull) return RTB_BAD_VALUE;
-    std::vector<ReplaySeg> segs(n_beams);
-    uint64_t tiles = 0;
+    std::vector<ReplaySeg> segs;
+    std::vector<SmallSeg> small;
+    small.reserve(n_beams);
+    uint64_t tiles = 0, covered = 0, end = 0;
     for (int b = 0; b < n_beams; ++b) {
+        const uint64_t first = h_beams[b].first_ray;
         const uint32_t nr = (uint32_t)h_beams[b].n_rays;
-        segs[b] = ReplaySeg{h_beams[b].first_ray, nr, nr, 0, 0, (uint32_t)tiles, 0};
-        if (b > 0 && segs[b].start < segs[b - 1].start + segs[b - 1].n) return RTB_BAD_VALUE;
-        tiles += (nr + (uint64_t)kTile - 1) / kTile;
+        if (first < end) return RTB_BAD_VALUE;
+        end = first + nr;
+        covered += nr;
+        if (nr == 0) continue;
+        if (nr <= (uint32_t)kSmallSeg) {
+            small.push_back(SmallSeg{first, nr, 0});
+        } else {
+            segs.push_back(ReplaySeg{first, nr, nr, 0, 0, (uint32_t)tiles, 0});
+            tiles += (nr + (uint64_t)kTile - 1) / kTile;
+        }
     }
+    std::vector<uint64_t> starts(covered < n ? n_beams : 0);
+    for (size_t b = 0; b < starts.size(); ++b) starts[b] = h_beams[b].first_ray;
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t o_any = 0, o_segs = 256, o_lost = o_segs + al(n_beams * sizeof(ReplaySeg)),
-                 o_stage = o_lost + al(tiles * 4), o_front = o_stage + al(tiles * kTile), o_back = o_front + al(n * 4);
+    const uint64_t listed = segs.empty() ? 0 : segs.back().start + segs.back().n;
+    const size_t o_any = 0, o_segs = 256, o_small = o_segs + al(segs.size() * sizeof(ReplaySeg)),
+                 o_starts = o_small + al(small.size() * sizeof(SmallSeg)),
+                 o_lost = o_starts + al(starts.size() * sizeof(uint64_t)), o_stage = o_lost + al(tiles * 4),
+                 o_front = o_stage + al(tiles * kTile), o_back = o_front + al(listed * 4);
     DevBuf buf;
-    int s = buf.alloc(o_back + al(n * 4), st);
+    int s = buf.alloc(o_back + al(listed * 4), st);
     if (s != RTB_OK) return s;
     char* p = buf.as<char>();
+    if (!starts.empty()) {
+        uint64_t* d = reinterpret_cast<uint64_t*>(p + o_starts);
+        RTB_CUDA_TRY(cudaMemcpyAsync(d, starts.data(), starts.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+        k_iota<<<grid_for(n, 256, 8), 256, 0, st>>>(n, d, (int)starts.size(), order);
+    }
+    if (!small.empty()) {
+        SmallSeg* d = reinterpret_cast<SmallSeg*>(p + o_small);
+        RTB_CUDA_TRY(cudaMemcpyAsync(d, small.data(), small.size() * sizeof(SmallSeg), cudaMemcpyHostToDevice, st));
+        k_replay_small<<<grid_for(small.size(), kSmallWarps, 8), 32 * kSmallWarps, 0, st>>>(
+            d, (int)small.size(), n_stages, rays.lost_stage, order);
+    }
+    RTB_CUDA_TRY(cudaGetLastError());
+    if (segs.empty()) return RTB_OK;
     Replay r;
     r.segs = reinterpret_cast<ReplaySeg*>(p + o_segs);
-    r.n_segs = n_beams;
+    r.n_segs = (int)segs.size();
     r.n_stages = n_stages;
     r.n_tiles = (uint32_t)tiles;
-    r.n = n;
     r.lost_stage = rays.lost_stage;
     r.order = order;
     r.stage = reinterpret_cast<uint8_t*>(p + o_stage);
@@ -376,11 +493,11 @@ int reference_order(const DevBeam* h_beams, int n_beams, int n_stages, const Dev
     r.back = reinterpret_cast<uint32_t*>(p + o_back);
     r.any = reinterpret_cast<unsigned*>(p + o_any);
     RTB_CUDA_TRY(cudaMemsetAsync(r.any, 0, 256, st));
-    RTB_CUDA_TRY(cudaMemcpyAsync(r.segs, segs.data(), n_beams * sizeof(ReplaySeg), cudaMemcpyHostToDevice, st));
+    RTB_CUDA_TRY(cudaMemcpyAsync(r.segs, segs.data(), segs.size() * sizeof(ReplaySeg), cudaMemcpyHostToDevice, st));
     int per_sm = 0;
     RTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_replay, kReplayThreads, 0));
     // no more blocks than tiles: the barriers cost by the block
-    unsigned blocks = grid_for(n, kTile, per_sm < 4 ? per_sm : 4);
+    unsigned blocks = grid_for(tiles, 1, per_sm < 4 ? per_sm : 4);
     void* args[] = {&r};
     RTB_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_replay), dim3(blocks),
                                              dim3(kReplayThreads), args, 0, st));
