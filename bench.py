@@ -277,6 +277,17 @@ def reference_arm(args):
     print(json.dumps(line), flush=True)
 
 
+def host_kernel(names, fp64: bool, specialize) -> str:
+    """The kernel rtb_trace_host launches, of `names` (compiled for the scheme,
+    for any scheme): the compiled one only in FP64, once `specialize` -- the
+    call a user makes ahead of one-shot traces -- has compiled it; mixed host
+    traces run the kernel for any scheme."""
+    if not fp64:
+        return names[1]
+    status, note = specialize()
+    return names[0] if status == 0 else f"{names[1]} ({note})"
+
+
 def main():
     args = parse()
     if args.impl == "reference":
@@ -592,10 +603,7 @@ def main():
         h = E.PinnedRays(n)
         src_cpu = {f: getattr(rays_in, f).cpu().numpy() for f in E.FIELDS}
         o = mk(ffi.ENGINE_FUSED, head_prec)
-        # the kernel compiled for the scheme (cached from the plan above;
-        # rtb_specialize is the call a user makes ahead of one-shot traces)
-        st_s, note = E.specialize(surf, FIXES, o.precision)
-        spec = KERNELS[head_prec][0] if st_s == ffi.OK else KERNELS[head_prec][1] + f" ({note})"
+        spec = host_kernel(KERNELS[head_prec], head_prec == ffi.FP64, lambda: E.specialize(surf, FIXES, o.precision))
         times = []
         for it in range(2 + max(1, args.steps // 3)):
             for f in E.FIELDS:
