@@ -100,6 +100,20 @@ __host__ __device__ constexpr unsigned scheme_bytes(int n_surfaces) {
     return (kSchemeHeader + (unsigned)n_surfaces * (unsigned)sizeof(DevSurface) + 15u) / 16u * 16u;
 }
 
+// Whether this code is compiled for any scheme, or at run time for one
+// (jit.cpp).
+#ifdef __CUDACC_RTC__
+constexpr bool kAnyScheme = false;
+#else
+constexpr bool kAnyScheme = true;
+#endif
+// Where the fused kernels' tables lie in shared memory, after the scheme: in
+// the kernels for any scheme at a fixed offset, which keeps registers free (an
+// offset by the number of surfaces cost C4's 4e6 rays 0.5 %, MIXED32 on C1 2 %).
+__host__ __device__ constexpr unsigned scheme_room(bool any_scheme, int n_surfaces) {
+    return scheme_bytes(any_scheme ? RTB_MAX_SURFACES : n_surfaces);
+}
+
 // Beam table on the device (first ray and orders of each beam).
 struct DevBeam {
     uint64_t first_ray;

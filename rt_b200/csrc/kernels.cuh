@@ -26,13 +26,13 @@ struct FrameArgs {
 };
 
 #ifndef __CUDACC_RTC__
-// Size of the dynamic shared memory the fused kernels use, and the size that
-// decides whether a scheme's tables fit a block: that of a full scheme,
-// whatever its number of surfaces.
-inline size_t fused_smem_bytes(int n_surfaces, int n_knots) {
-    return scheme_bytes(n_surfaces) + sizeof(double) * (size_t)n_knots;
+// Size of the dynamic shared memory the fused kernels use (any_scheme: those
+// not compiled for a scheme), and the size that decides whether a scheme's
+// tables fit a block: that of a full scheme, whatever its number of surfaces.
+inline size_t fused_smem_bytes(bool any_scheme, int n_surfaces, int n_knots) {
+    return scheme_room(any_scheme, n_surfaces) + sizeof(double) * (size_t)n_knots;
 }
-inline size_t fused_smem_limit(int n_knots) { return fused_smem_bytes(RTB_MAX_SURFACES, n_knots); }
+inline size_t fused_smem_limit(int n_knots) { return fused_smem_bytes(true, RTB_MAX_SURFACES, n_knots); }
 #endif
 
 // Scheduling of the persistent fused kernels: `next` is a counter of tiles

@@ -249,8 +249,9 @@ __device__ __forceinline__ void fused_mixed32(const DevScheme* __restrict__ g_sc
                                               FrameArgs frame, TileSched ts) {
     const double* s_knots;
     const DevScheme* sch = stage_scheme<Surfaces::kBaked>(g_sch, knots, ts, s_knots);
-    const int n_stages = 3 * ts.n_surfaces;
-    RowLoop rows(ts, in.n, warp_row_buffer<Row32>(ts.n_surfaces, ts.n_knots), (unsigned)sizeof(Row32), err);
+    const int n_stages = 3 * (kAnyScheme ? sch->n_surfaces : ts.n_surfaces);
+    RowLoop rows(ts, in.n, warp_row_buffer<Row32>(ts.n_surfaces, kAnyScheme ? sch->n_knots : ts.n_knots),
+                 (unsigned)sizeof(Row32), err);
     const int lane = threadIdx.x & 31;
     BeamCursor cur;
     EventCounter events;
@@ -334,11 +335,15 @@ __device__ __forceinline__ void fused_mixed32(const DevScheme* __restrict__ g_sc
         } else if (valid && (rows.packed || in.flag != out.flag)) {
             out.flag[oi] = f;
         }
-        events.add(ev, key, counts);
-        if (ts.rpt == 1) events.flush(counts);  // a small trace: not all warps' at the end
+        if (kAnyScheme) {
+            count_event(ev, key, counts);
+        } else {
+            events.add(ev, key, counts);
+            if (ts.rpt == 1) events.flush(counts);  // a small trace: not all warps' at the end
+        }
         if (frame.counts) frame_add<false>(good, outX, outY, frame);
     }
-    events.flush(counts);
+    if (!kAnyScheme) events.flush(counts);
 }
 
 }  // namespace rtb

@@ -113,7 +113,7 @@ extern "C" RTB_API int rtb_trace_out_noalloc(const rtb_surface* surfaces, size_t
     const Layout l = layout(n_knots, n_beams, n_beams * ns1);
     if (l.total > RTB_NOALLOC_SCRATCH_BYTES) return RTB_BAD_VALUE;
     if (fused_smem_limit((int)n_knots) > (size_t)engine().max_smem_optin) return RTB_BAD_VALUE;
-    const size_t smem = fused_smem_bytes((int)n_surfaces, (int)n_knots);
+    const size_t smem = fused_smem_bytes(true, (int)n_surfaces, (int)n_knots);
     std::memcpy(h_stage, &h_scheme, sizeof(DevScheme));
     DevBeam* beams_h = reinterpret_cast<DevBeam*>(h_stage + l.beams);
     uint64_t prev_end = 0;

@@ -189,7 +189,7 @@ __host__ __device__ constexpr size_t row_buffers_bytes(int threads) {
 template <class Row>
 __device__ __forceinline__ unsigned char* warp_row_buffer(int n_surfaces, int n_knots) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const size_t base = (scheme_bytes(n_surfaces) + sizeof(double) * (size_t)n_knots + 127) / 128 * 128;
+    const size_t base = (scheme_room(kAnyScheme, n_surfaces) + sizeof(double) * (size_t)n_knots + 127) / 128 * 128;
     return smem + base + (size_t)(threadIdx.x >> 5) * row_buffer_bytes<Row>();
 }
 

@@ -148,7 +148,7 @@ int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_
             return (b + 127) / 128 * 128 + (m32 ? row_buffers_bytes<Row32>(threads) : row_buffers_bytes<Row64>(threads));
         };
         if (with_rows(fused_smem_limit(ps.sch.n_knots)) > (size_t)engine().max_smem_optin) return RTB_BAD_VALUE;
-        const size_t smem = with_rows(fused_smem_bytes(ps.sch.n_surfaces, ps.sch.n_knots));
+        const size_t smem = with_rows(fused_smem_bytes(!ps.scheme_kernel, ps.sch.n_surfaces, ps.sch.n_knots));
         const void* kern = ps.scheme_kernel ? ps.scheme_kernel
                            : m32           ? reinterpret_cast<const void*>(k_fused_mixed32)
                            : mixed         ? reinterpret_cast<const void*>(k_fused_mixed)
