@@ -111,15 +111,19 @@ int gen_beams(const rtb_beam* beams, size_t n_beams, size_t n_rays, std::vector<
 
 // Rows of 32 rays that a warp (mixed) or rays that a thread (FP64) takes at a
 // time.  More of them amortise the tile counter, whose one address serves all
-// warps; fewer spread a small trace over the chip.  On C1 in a plan, ms at 1 /
-// 2 / 4 rows: mixed 2e5 rays (1.3 rows per resident warp) 0.051 / 0.054 /
-// 0.071, 6e5 (4) 0.076 / 0.075 / 0.087, 2e6 (13) 0.182 / 0.148 / 0.138, 1e8
-// 5.73 / 3.87 / 3.87; FP64, whose blocks share a tile and step through the
-// surfaces together, 2e5 0.075 / 0.079 / 0.102, 2e7 2.88 / 2.89 / 2.92.
+// warps, and bound traces of few surfaces; fewer spread a small trace over the
+// chip and leave less of the last round idle, and bound long ones.  Mixed
+// plans, us at 1 / 2 / 3 / 4 rows:
+//   rows per resident warp    2                   13                    40                      132
+//   C0                 36/ 35/ 37/ 37     103/ 87/ 86/ 86    294/ 246/ 236/ 236     1111/ 839/ 750/ 738
+//   C1                 40/ 42/ 50/ 59     124/123/125/129    308/ 293/ 289/ 294      959/ 873/ 850/ 847
+//   12 aspheres        89/ 99/114/134     414/419/418/430   1161/1165/1177/1183     3785/3782/3785/3793
+//   22 of all kinds    43/ 49/ 53/ 62     125/123/127/135    327/ 299/ 306/ 307     1041/ 922/ 913/ 910
+// FP64, us at 1 / 2 / 4, C1 in a plan: 2e5 rays 75/79/102, 2e7 2880/2890/2920.
 int default_rpt(int precision, uint64_t n_rays) {
     if (precision == RTB_FP64) return 1;
     const uint64_t warps = (uint64_t)engine().sm_count * 32, rows = n_rays / 32;
-    return rows < 2 * warps ? 1 : rows < 8 * warps ? 2 : 4;
+    return rows < 2 * warps ? 1 : rows < 16 * warps ? 2 : rows < 96 * warps ? 3 : 4;
 }
 
 int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_trace_opts& o, const DevRays& in,
