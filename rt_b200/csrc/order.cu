@@ -506,18 +506,21 @@ int reference_order(const DevBeam* h_beams, int n_beams, int n_stages, const Dev
 
 // Beam::Rearrange over host arrays: the lost rays are counted first; none, and
 // nothing moves.  A swap touches two rays, so where few are lost the kernel
-// swaps them in the host arrays themselves when those are library vectors (C0,
-// 1e5 rays of which 1 % lost: 13 us against 0.22 ms of copies); many are swapped in device copies, 57
-// bytes a ray each way at the link's full rate.
-constexpr size_t kSwapInPlace = 64;  // at most one ray in this many lost
+// swaps them in the host arrays themselves when those are library vectors;
+// many are swapped in device copies, 57 bytes a ray each way at the link's full
+// rate.  In place against copies, us: 1e4 rays of which 1/64 / 1/4 lost 91/148
+// and 96/147; 1e5 of which 1/64 / 1/8 / 1/4 133/343, 273/350 and 363/356; 1e6 of
+// which 1/128 / 1/64 / 1/32 902/2193, 1553/2221 and 2264/2228.
+constexpr size_t kSwapInPlace = 64;       // at most one ray in this many lost,
+constexpr size_t kSwapInPlaceRays = 2048;  // or no more than this
 int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out, cudaStream_t st) {
     Work w;
     int s = w.init(ng, 1, st);
     if (s != RTB_OK) return s;
-    bool vectors = in_host_vector(flag, ng, 1);
+    bool vectors = true;  // the seven arrays: the flags may lie elsewhere (the reference's do)
     char* dflag = flag;
     DevBuf fbuf, buf;
-    if (!vectors) {
+    if (!in_host_vector(flag, ng, 1)) {
         if ((s = fbuf.alloc(ng, st)) != RTB_OK) return s;
         dflag = fbuf.as<char>();
         RTB_CUDA_TRY(cudaMemcpyAsync(dflag, flag, ng, cudaMemcpyHostToDevice, st));
@@ -536,7 +539,7 @@ int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out,
         return RTB_OK;
     }
     Arr7 arr;
-    const bool in_place = lost <= ng / kSwapInPlace;
+    const bool in_place = lost <= ng / kSwapInPlace || lost <= kSwapInPlaceRays;
     for (int i = 0; i < 7; ++i) {
         vectors = vectors && in_host_vector(host[i], ng * sizeof(double), sizeof(double));
         for (int j = 0; j < i; ++j)  // an array given twice is swapped once
@@ -544,6 +547,13 @@ int rearrange_host(size_t ng, double* const host[7], char* flag, size_t* ng_out,
     }
     const bool copies = !(vectors && in_place);
     if (copies && (s = buf.alloc(7 * ng * sizeof(double), st)) != RTB_OK) return s;
+    // the flags too: many single bytes stored over the link took 0.25 ms of 2.45
+    // (1e6 rays, 40 % lost)
+    if (copies && dflag == flag) {
+        if ((s = fbuf.alloc(ng, st)) != RTB_OK) return s;
+        dflag = fbuf.as<char>();
+        RTB_CUDA_TRY(cudaMemcpyAsync(dflag, flag, ng, cudaMemcpyHostToDevice, st));
+    }
     for (int i = 0; i < 7; ++i) {
         arr.a[i] = copies ? buf.as<double>() + (size_t)i * ng : host[i];
         if (copies) RTB_CUDA_TRY(cudaMemcpyAsync(arr.a[i], host[i], ng * sizeof(double), cudaMemcpyHostToDevice, st));
