@@ -96,12 +96,15 @@ __device__ __forceinline__ unsigned slot_hash(unsigned long long k) {
     return h ^ (h >> 15);
 }
 
-// The slot of k in a table, taken if k is not there; -1 when `most` are taken.
+// The slot of k in a table, taken if k is not there; -1 when `most` are taken
+// (a key too many is not put in: in a full table every further look-up would
+// walk all of it, 2000 values of 4e6 rays 50 us).
 __device__ __forceinline__ int slot_of(unsigned long long* keys, unsigned mask, unsigned* used, unsigned most,
                                        unsigned long long k) {
     for (unsigned i = slot_hash(k) & mask, tries = 0; tries <= mask; i = (i + 1) & mask, ++tries) {
         unsigned long long at = *(volatile unsigned long long*)(keys + i);
         if (at == kNoKey) {
+            if (*(volatile unsigned*)used + 1u >= most) return -1;
             at = atomicCAS(keys + i, kNoKey, k);
             if (at == kNoKey) return atomicAdd(used, 1u) + 1u < most ? (int)i : -1;
         }
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(kDistinctThreads) k_distinct(const double* lam
         if (threadIdx.x == 0) *(volatile unsigned*)t.few = 0u;
         return;
     }
+    if (!*(volatile unsigned*)t.few) return;
     for (int j = threadIdx.x; j < kSlots; j += blockDim.x) {
         if (key[j] == kNoKey) continue;
         const int s = slot_of(t.key, kGlobalSlots - 1, t.used, kMaxDistinct, key[j]);
