@@ -250,7 +250,9 @@ RTB_API int rtb_grating_energy_distr(size_t n, const double* lambda, long order,
                              double rule_stop, double* energy_distr);
 
 /* rt_engine_free_vector / rt_engine_alocate_vector (rt_engine_func.h:84-86):
- * page-locked host vectors, so the drop-in copies run at full PCIe rate. */
+ * page-locked host vectors.  The calls on host arrays read and write them in
+ * place over the link, where their elements are aligned; rtb_free_vector ends
+ * that, so free them by no other call. */
 RTB_API void rtb_free_vector(double* data);
 RTB_API double* rtb_alocate_vector(size_t n_elem);
 
@@ -607,8 +609,8 @@ RTB_API int rtb_adjoint_forward(rtb_adjoint* ctx, const double* theta, const rtb
                                 char* flag, rtb_trace_stats* stats, void* stream);
 /* grad[j] = sum over rays of gX * dX/dtheta_j + gY * dY/dtheta_j for the last
  * forward (gX, gY device, n_rays; grad host, n_params).  Deterministic.  One
- * reverse sweep per ray through the surfaces, each surface recomputed from its
- * checkpoint; with the environment variable RTB_ADJOINT_BACKWARD=passes, the
+ * reverse sweep per ray through the surfaces, between their checkpoints;
+ * with the environment variable RTB_ADJOINT_BACKWARD=passes, the
  * same gradient (to rounding) by forward-mode dual-number passes. */
 RTB_API int rtb_adjoint_backward(rtb_adjoint* ctx, const double* gX, const double* gY, double* grad, void* stream);
 /* Forward-mode sensitivities of the last forward along dtheta (host, n_params):

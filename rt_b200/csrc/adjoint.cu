@@ -6,9 +6,10 @@
 // bits), storing each ray's state at the input of every surface; compiled
 // for the scheme's structure like the backward.
 //
-// Backward (adjoint_rev.cuh): per ray, surfaces last to first, each surface
-// recomputed from its checkpoint and its adjoint carried back through its
-// stages in one reverse sweep (ray_rev.cuh); the kernel compiled for the
+// Backward (adjoint_rev.cuh): per ray, surfaces last to first, the adjoint of
+// a surface's output state (the next checkpoint; the last surface is
+// recomputed) carried back through its stages to its input state (its
+// checkpoint) in one reverse sweep (ray_rev.cuh); the kernel compiled for the
 // scheme's structure when NVRTC is there (jit.cpp, rtb_adj_reverse_scheme;
 // RTB_SPECIALIZE=0 keeps the generic k_adj_reverse), its sums reproducible.
 //

@@ -89,10 +89,11 @@ struct AdjShape {
 // they leave at different steps, and before the last normalisation: without
 // that each group of lanes ran the rest of the scheme by itself (C4: the
 // detector's plane took the instructions of three surfaces at 9 lanes of 32),
-// 0.39 ms against 0.36 for 2e6 rays.  The fused FP64 kernel, whose blocks meet
-// after every surface, and the reverse sweep, whose warps do, lose by it
-// (2.87 -> 2.96 and 0.70 -> 0.75 ms): there the groups hide each other's
-// latency within the surface.
+// 443 us against 357 for 2e6 rays, 48.5 against 40.2 for 2e5.  The fused FP64
+// kernel compiled for its scheme loses by the same meeting (C1, 2e7 rays 2.77 ->
+// 2.94 ms; C4 2.57 -> 2.63; 2e6 rays 0.339 -> 0.353), and so does the reverse
+// sweep before its parameter sums (C4, 2e6 rays 476 -> 479 us; 2e5 54.2 -> 55.9):
+// there the groups hide each other's latency.
 template <class Sh>
 __device__ __forceinline__ int fwd_surface(const AdjArgs& a, int k, size_t i, int b, double lam, unsigned* err,
                                            unsigned& live, f64::Ray& r) {

@@ -1,9 +1,9 @@
 // engine.cu -- C ABI: engine state, scheme preparation and the drop-in calls
 // of common-lib/rt_engine_func.h (host arrays in and out, synchronous).
 //
-// Each drop-in call copies the arrays it reads to the device, runs one
-// kernel and copies back what the reference's call returns; the copies and
-// the kernel are ordered on the library stream, the temporaries come from the
+// Each drop-in call runs one kernel on the caller's arrays, library vectors in
+// place over the link, others copied to the device before it and back after it
+// (HostArrays); the copies and the kernel are ordered on the library stream, the temporaries come from the
 // stream-ordered pool (no cudaMalloc/cudaFree per call as in
 // rt_cuda_engine_common.cu:72-155).
 #include <algorithm>
@@ -560,6 +560,11 @@ struct HostArrays {
     // enough to keep it busy, and with more of them all the loads go before
     // all the stores, one direction at a time: the transform of 1e5 rays took
     // 171 us with a thread per ray, 141 at 148 blocks, 126 at 16 to 48, 131 at 8.
+    // Kernels of more arithmetic are bound by the link too: at 48 blocks / 148 /
+    // no limit the intersection with C1's asphere took 147/142/160, with its
+    // toric 146/143/163, refraction with a glass table 165/167/182; aspheres of
+    // twice to five times the curvature, whose root takes long, 187/196/188,
+    // 297/276/279, 285/295/264 and 204/194/191.
     static constexpr unsigned kLinkBlocks = 48;
     unsigned grid(size_t count) const {
         bool mapped = false;
@@ -996,6 +1001,8 @@ extern "C" int rtb_grating_energy_distr(size_t n, const double* lambda, long ord
     g.add(lambda, n, true, false);
     g.add(energy_distr, n, true, true);
     if ((st = g.open(false)) != RTB_OK) return st;
+    // arithmetic, not the link, bounds this one: 1e5 values 397 us, 648 at 148
+    // blocks and 1816 at HostArrays' 48
     k_grating_energy<<<grid_for(n, 256, 8), 256, 0, s>>>(n, g.d(0), (long long)order, blaze_angle, alpha, gamma,
                                                           gr_const, rule_start, rule_stop, g.d(1));
     return g.close();

@@ -292,13 +292,15 @@ int rtb_plan_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
     // the coherent tracing order and a copy of the rays in that order, once
     // (index order for plans beyond 2^32 rays).  The rays of a beam are
     // grouped by wavelength within chunks of 2^20 consecutive rays for the
-    // mixed kernel and of the whole beam (up to 2^30) for the FP64 kernel:
-    // the best of 2^11..2^30 for each on C1 (mixed: 5.24 ms at 2^20, 5.36
-    // whole beams, 5.65 at 2^11; FP64: 24.7 ms whole beams, 25.1 at 2^20).
-    // Outputs are stored at the rays' indices, 8 bytes apart per lane, which
-    // costs the mixed kernel 0.8 ms of its 5.3 on C1 against coalesced stores;
-    // chunks small enough to stage a block's stores in shared memory lose
-    // more in coherence than that.
+    // mixed kernel and of the whole beam (up to 2^30) for the FP64 kernel,
+    // which serves outputs at the rays' indices best.  C1, 1e8 rays, ms with
+    // outputs by index / by slot: mixed 2^11 4.45/4.35, 2^14 4.29/4.03, 2^17
+    // 4.08/3.72, 2^20 4.05/3.59, whole beams 4.30/3.53; FP64 2^20 13.54/13.27,
+    // whole beams 13.27/12.94.  C3's 512 uneven beams (1.8e7 rays) take
+    // the mixed kernel 0.76 by index whatever the chunk, 0.74 by slot
+    // at 2^11 and 0.70 from 2^20 on.  Stores by index, 8 bytes apart per lane,
+    // thus cost C1 13 % and C3 8 %; chunks small enough to stage a block's stores
+    // in shared memory (2^11) lose as much in coherence.
     // The order is beam-major (k_order_keys): the slots of beam b are the
     // range of its ray indices, so a kernel reading rows finds a ray's beam
     // from its slot.  The mixed kernels read the ordered copy as row blocks of 32 rays

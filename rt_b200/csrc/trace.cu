@@ -119,7 +119,8 @@ int gen_beams(const rtb_beam* beams, size_t n_beams, size_t n_rays, std::vector<
 //   C1                 40/ 42/ 50/ 59     124/123/125/129    308/ 293/ 289/ 294      959/ 873/ 850/ 847
 //   12 aspheres        89/ 99/114/134     414/419/418/430   1161/1165/1177/1183     3785/3782/3785/3793
 //   22 of all kinds    43/ 49/ 53/ 62     125/123/127/135    327/ 299/ 306/ 307     1041/ 922/ 913/ 910
-// FP64, us at 1 / 2 / 4, C1 in a plan: 2e5 rays 75/79/102, 2e7 2880/2890/2920.
+// FP64 plans, whose blocks meet at every tile, us at 1 / 2 / 4 rays a thread: C1
+// 2e5 rays 61/63/87, 2e7 2774/2950/3134; 12 aspheres 120/132/168, 7341/7527/7668.
 int default_rpt(int precision, uint64_t n_rays) {
     if (precision == RTB_FP64) return 1;
     const uint64_t warps = (uint64_t)engine().sm_count * 32, rows = n_rays / 32;
@@ -333,11 +334,14 @@ int rtb_rearrange(size_t* n_good, double* X, double* Y, double* Z, double* cX, d
 
 namespace rtb {
 
-// Whether rtb_trace_host traces the arrays where they lie: all of them library
-// vectors (rtb_alocate_vector) apart from one another, the beams covering every
-// ray, and not so many rays that the copy engines' higher rate pays for the
-// first chunk's copy-in and the last one's copy-out, when only one direction
-// of the link is busy (kHostInPlace).
+// Whether rtb_trace_host traces the arrays where they lie: all of them aligned
+// library vectors (rtb_alocate_vector) apart from one another, the beams
+// covering every ray, and no more rays than kHostInPlace, up to where it was
+// measured against the chunks below for short and long schemes.  In place /
+// chunks, ms: C1 FP64 1e6 rays 1.45/2.46, 8e6 10.4/23.4, 1.6e7 20.7/27.8, mixed
+// 8e6 9.3/12.6, 1.6e7 18.5/22.3; 20 aspheres FP64 1e5 0.49/0.68, 1e6 2.03/3.02,
+// 1.6e7 27.9/28.6; 31 aspheres 1e6 2.86/3.43, 8e6 20.2/36.8.  (Beyond, C1 at
+// 6.4e7 rays: FP64 81/115, mixed 73/90.)
 constexpr uint64_t kHostInPlace = 1ull << 24;
 static bool host_in_place(const rtb_rays* h, const std::vector<DevBeam>& db) {
     const uint64_t n = h->n;
@@ -369,7 +373,11 @@ static bool host_in_place(const rtb_rays* h, const std::vector<DevBeam>& db) {
 // lanes come to the stores in groups, which the link carries as partial lines
 // (C1, 1e6 rays, X and Y back 2573 us, all of the state back 4280; the kernels
 // for any scheme 1362 and 1680).  Meeting before the stores cures it too but
-// costs plans 1.2 %, and the link is the bound with either kernel.
+// costs plans 1.2 %.  The chunks take the kernel for any scheme as well: the two
+// differ in the last bits, and an array's results depend neither on where it
+// lies nor on whether a plan has compiled its scheme.  Nothing is lost by it,
+// the link is the bound with either (C1 mixed through the chunks, kernel for any
+// scheme / compiled: 1e5 rays 384/422 us, 1e6 1750/1744, 5e7 59.5/60.6 ms).
 //
 // Other arrays and more rays: chunks of rays cycle through two device
 // buffers on two streams, so that the copy-in of one chunk, the trace of the
