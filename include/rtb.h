@@ -381,7 +381,7 @@ typedef struct {
  * that frame (the plan never clears it).  block_size / rays_per_thread 0
  * take the configuration an earlier rtb_plan_autotune chose for the same
  * scheme, precision, frame use and ray count in this process, else the
- * defaults (256 x 1 to 4, by precision and ray count).  A plan launches a copy of the fused kernel of its
+ * defaults (256 x 1, 2 or 4, by precision, surfaces and ray count).  A plan launches a copy of the fused kernel of its
  * precision compiled for its scheme's structure with NVRTC when the plan is
  * made (the same arithmetic -- for RTB_FP64 the same IEEE operations, bit
  * for bit -- without the per-surface branching on surface kind, type and

@@ -224,7 +224,8 @@ int coherent_order(const GenBeam* d_beams, int n_beams, uint64_t n, const DevRay
                    int chunk_shift, cudaStream_t st);
 // The launch configuration of a trace that names none.
 constexpr int kDefaultBlock = 256;
-int default_rpt(int precision, uint64_t n_rays);
+constexpr int kManySurfaces = 10;  // C1's seven surfaces lie below it, the schemes of 12 and more measured above
+int default_rpt(int precision, int n_surfaces, uint64_t n_rays);
 // Status and statistics from the per-(beam, stage) counts.
 int trace_result(const PreparedScheme& ps, const unsigned long long* counts, unsigned err, int n_beams,
                  rtb_trace_stats* stats);

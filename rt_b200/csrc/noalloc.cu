@@ -88,7 +88,7 @@ extern "C" RTB_API int rtb_trace_out_noalloc(const rtb_surface* surfaces, size_t
     // the launch configuration rtb_trace_out accepts (launch_trace)
     const int threads = (opts->block_size > 0) ? opts->block_size : 256;
     if (threads != 128 && threads != 256 && !(mixed && threads == 512)) return RTB_BAD_VALUE;
-    const int rpt = (opts->rays_per_thread > 0) ? opts->rays_per_thread : default_rpt(opts->precision, in->n);
+    const int rpt = (opts->rays_per_thread > 0) ? opts->rays_per_thread : default_rpt(opts->precision, (int)n_surfaces, in->n);
     if (rpt < 1 || rpt > 64) return RTB_BAD_VALUE;
     const size_t ns1 = 3 * n_surfaces + 1;
     if (layout(0, n_beams, n_beams * ns1).total > RTB_NOALLOC_SCRATCH_BYTES) return RTB_BAD_VALUE;

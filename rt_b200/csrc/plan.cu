@@ -241,7 +241,7 @@ int rtb_plan_create(const rtb_surface* surfaces, size_t n_surfaces, const rtb_be
         delete p;
         return st;
     }
-    p->rpt = default_rpt(opts->precision, p->n_rays);
+    p->rpt = default_rpt(opts->precision, p->ps.sch.n_surfaces, p->n_rays);
     if (opts->block_size > 0 || opts->rays_per_thread > 0) {
         if (opts->block_size > 0) p->block = opts->block_size;
         if (opts->rays_per_thread > 0) p->rpt = opts->rays_per_thread;

@@ -111,20 +111,25 @@ int gen_beams(const rtb_beam* beams, size_t n_beams, size_t n_rays, std::vector<
 
 // Rows of 32 rays that a warp (mixed) or rays that a thread (FP64) takes at a
 // time.  More of them amortise the tile counter, whose one address serves all
-// warps, and bound traces of few surfaces; fewer spread a small trace over the
-// chip and leave less of the last round idle, and bound long ones.  Mixed
-// plans, us at 1 / 2 / 3 / 4 rows:
-//   rows per resident warp    2                   13                    40                      132
-//   C0                 36/ 35/ 37/ 37     103/ 87/ 86/ 86    294/ 246/ 236/ 236     1111/ 839/ 750/ 738
-//   C1                 40/ 42/ 50/ 59     124/123/125/129    308/ 293/ 289/ 294      959/ 873/ 850/ 847
-//   12 aspheres        89/ 99/114/134     414/419/418/430   1161/1165/1177/1183     3785/3782/3785/3793
-//   22 of all kinds    43/ 49/ 53/ 62     125/123/127/135    327/ 299/ 306/ 307     1041/ 922/ 913/ 910
+// warps beside the frame's pixels: that bounds schemes of few surfaces.  Fewer
+// spread a small trace over the chip and leave less of the last round idle:
+// that bounds schemes of many.  Mixed plans, us at 1 / 2 / 4 rows for 2 rows per
+// resident warp (no frame), at 2 / 3 / 4 for more (with a frame but for the
+// first two lines):
+//                                        2           13             33              53
+//   C0                              36/ 35/ 37    87/  86/  86                 401/ 383/ 382 (66 rows)
+//   C1                              40/ 42/ 59   123/ 124/ 128   247/ 247/ 249   373/ 370/ 370
+//   C1, frame                                    162/ 146/ 139   327/ 284/ 271   477/ 416/ 394
+//   C1 and 8 lens surfaces                       258/ 271/ 281   541/ 553/ 565   822/ 831/ 840
+//   12 aspheres                     89/ 99/134   436/ 455/ 458  1011/1023/1031  1588/1600/1619
+//   20 aspheres                    247/279/393  1217/1268/1330  2922/2971/2977  4612/4644/4709
+//   22 surfaces of all kinds        43/ 49/ 62   123/ 128/ 136   260/ 265/ 270   397/ 396/ 399
 // FP64 plans, whose blocks meet at every tile, us at 1 / 2 / 4 rays a thread: C1
 // 2e5 rays 61/63/87, 2e7 2774/2950/3134; 12 aspheres 120/132/168, 7341/7527/7668.
-int default_rpt(int precision, uint64_t n_rays) {
+int default_rpt(int precision, int n_surfaces, uint64_t n_rays) {
     if (precision == RTB_FP64) return 1;
     const uint64_t warps = (uint64_t)engine().sm_count * 32, rows = n_rays / 32;
-    return rows < 2 * warps ? 1 : rows < 16 * warps ? 2 : rows < 96 * warps ? 3 : 4;
+    return rows < 2 * warps ? 1 : rows < 8 * warps || n_surfaces >= kManySurfaces ? 2 : 4;
 }
 
 int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_trace_opts& o, const DevRays& in,
@@ -146,7 +151,7 @@ int launch_trace(const PreparedScheme& ps, TraceArgs& a, int n_beams, const rtb_
         if (rows && !mixed) return RTB_BAD_VALUE;
         const int threads = (o.block_size > 0) ? o.block_size : kDefaultBlock;
         if (threads != 128 && threads != 256 && !(mixed && threads == 512)) return RTB_BAD_VALUE;
-        const int rpt = (o.rays_per_thread > 0) ? o.rays_per_thread : default_rpt(o.precision, in.n);
+        const int rpt = (o.rays_per_thread > 0) ? o.rays_per_thread : default_rpt(o.precision, ps.sch.n_surfaces, in.n);
         if (rpt < 1 || rpt > 64) return RTB_BAD_VALUE;
         auto with_rows = [&](size_t b) {
             if (!rows) return b;

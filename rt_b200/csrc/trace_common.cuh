@@ -101,7 +101,7 @@ __device__ __forceinline__ void count_event(bool ev, int key, unsigned long long
 // kernel, slower per row, gains nothing (1 % slower) and counts row by row, and
 // so do the mixed kernels for any scheme, where the two registers it keeps are
 // spilled: one-shot traces of 4e6 rays, C1 483 us with it and 452 without, C4
-// 320 and 306, C0 187 and 182.
+// 320 and 306, C0 187 and 181.
 struct EventCounter {
     int key = -1;
     unsigned n = 0;

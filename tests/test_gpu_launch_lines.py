@@ -1,6 +1,6 @@
-"""The launch configuration a mixed trace takes by itself, at the ray counts
-where it changes beyond those of test_gpu_launch (GPU test): every ray traced
-once, with the results of an explicit configuration.
+"""The launch configuration a mixed trace takes by itself where the number of
+surfaces decides it (GPU test): every ray traced once, with the results of an
+explicit configuration.
 """
 import numpy as np
 import pytest
@@ -15,9 +15,12 @@ ROWS = 148 * 32     # rows of 32 rays, one per resident warp
 
 
 @pytest.mark.parametrize("precision", [ffi.MIXED, ffi.MIXED32])
-@pytest.mark.parametrize("n", [32 * 16 * ROWS - 5, 32 * 16 * ROWS, 32 * 96 * ROWS - 1, 32 * 96 * ROWS + 33])
-def test_default_configuration_traces_every_ray_once(precision, n):
-    surf = S.to_c(S.littrow_free(), E.spline_init).surfaces
+@pytest.mark.parametrize("surfaces", [9, 10, 32])
+@pytest.mark.parametrize("n", [32 * 2 * ROWS - 1, 32 * 2 * ROWS, 32 * 8 * ROWS - 7, 32 * 8 * ROWS + 33])
+def test_default_configuration_traces_every_ray_once(precision, surfaces, n):
+    idle = S.SurfaceSpec(ffi.AUX_CLASS, ffi.AUX_TYPE, distance=(0.0, 0.0, 0.0))
+    specs = S.littrow_free()
+    surf = S.to_c([idle] * (surfaces - len(specs)) + specs, E.spline_init).surfaces
     beams = [S.make_beam(0, n, 1, S.C0_RADIUS, (0.55, 0.55), 5)]
     results = []
     for block, rpt in ((0, 0), (128, 7)):
@@ -27,6 +30,8 @@ def test_default_configuration_traces_every_ray_once(precision, n):
         assert st == ffi.OK
         out = E.device_view(plan.rays()[1])
         assert stats.n_good == int((out["flag"] == 1).sum()) > 0
+        if not rpt:
+            assert plan.config()[1] == (1 if n < 64 * ROWS else 2 if n < 256 * ROWS or surfaces >= 10 else 4)
         results.append([out[f].clone() for f in ("flag", "lost_stage", "X", "Y")])
         torch.cuda.synchronize()
         plan.destroy()
