@@ -201,8 +201,10 @@ std::string scheme_source(const DevScheme& sch, int precision) {
     const bool bake = bake_values();
     const std::string S = bake ? "k_surfaces()[" : "sch->s[";
     const std::string F = bake ? "k_fixes" : "sch->fixes";
-    const std::string kBaked = bake ? "    static constexpr bool kBaked = true;\n"
-                                    : "    static constexpr bool kBaked = false;\n";
+    // schemes of many surfaces have no registers left for a counter (EventCounter)
+    const std::string kBaked = std::string("    static constexpr bool kBaked = ") + (bake ? "true" : "false") +
+                               ";\n    static constexpr bool kKeepsCounter = " +
+                               (sch.n_surfaces < kManySurfaces ? "true" : "false") + ";\n";
     if (precision == RTB_MIXED) {
         src = "#include \"mixed.cuh\"\n" + (bake ? surface_constants(sch) : std::string()) +
               "namespace rtb {\n"

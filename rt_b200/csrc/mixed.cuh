@@ -573,6 +573,7 @@ __device__ __forceinline__ int mx_surface(const DevSurface& s, int k, uint32_t f
 // surface's FixedShape in turn.
 struct RtSurfaces {
     static constexpr bool kBaked = false;
+    static constexpr bool kKeepsCounter = false;
     __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots, const BeamCtx& bc,
                                                double lam, mx::TableMemo& memo, mx::Ray& r, int& stage) {
         for (int k = 0; k < sch->n_surfaces && stage == -1; ++k)
@@ -669,15 +670,15 @@ __device__ __forceinline__ void fused_mixed(const DevScheme* __restrict__ g_sch,
         } else if (valid && (rows.packed || in.flag != out.flag)) {
             out.flag[oi] = f;
         }
-        if (kAnyScheme) {
-            count_event(ev, key, counts);
-        } else {
+        if (Surfaces::kKeepsCounter) {
             events.add(ev, key, counts);
             if (ts.rpt == 1) events.flush(counts);  // a small trace: not all warps' at the end
+        } else {
+            count_event(ev, key, counts);
         }
         if (frame.counts) frame_add<false>(good, outX, outY, frame);
     }
-    if (!kAnyScheme) events.flush(counts);
+    if (Surfaces::kKeepsCounter) events.flush(counts);
 }
 
 }  // namespace rtb

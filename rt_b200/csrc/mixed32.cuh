@@ -230,6 +230,7 @@ __device__ __forceinline__ int m32_surface(const DevSurface& s, int k, uint32_t 
 // FixedShape per surface).
 struct Rt32Surfaces {
     static constexpr bool kBaked = false;
+    static constexpr bool kKeepsCounter = false;
     __device__ __forceinline__ static void run(const DevScheme* sch, const double* knots, const BeamCtx& bc,
                                                const double* off0, double lam, mx::TableMemo& memo, m32::Ray& r,
                                                mx::Ray& q, int& stage) {
@@ -335,15 +336,15 @@ __device__ __forceinline__ void fused_mixed32(const DevScheme* __restrict__ g_sc
         } else if (valid && (rows.packed || in.flag != out.flag)) {
             out.flag[oi] = f;
         }
-        if (kAnyScheme) {
-            count_event(ev, key, counts);
-        } else {
+        if (Surfaces::kKeepsCounter) {
             events.add(ev, key, counts);
             if (ts.rpt == 1) events.flush(counts);  // a small trace: not all warps' at the end
+        } else {
+            count_event(ev, key, counts);
         }
         if (frame.counts) frame_add<false>(good, outX, outY, frame);
     }
-    if (!kAnyScheme) events.flush(counts);
+    if (Surfaces::kKeepsCounter) events.flush(counts);
 }
 
 }  // namespace rtb

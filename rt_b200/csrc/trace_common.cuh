@@ -99,9 +99,11 @@ __device__ __forceinline__ void count_event(bool ev, int key, unsigned long long
 // a single address bound schemes of few surfaces: C0 mixed, 6e6 rays in one
 // beam 0.216 -> 0.148 ms; C1, 1e8 rays in 31 beams 3.86 -> 3.72.  The FP64
 // kernel, slower per row, gains nothing (1 % slower) and counts row by row, and
-// so do the mixed kernels for any scheme, where the two registers it keeps are
-// spilled: one-shot traces of 4e6 rays, C1 483 us with it and 452 without, C4
-// 320 and 306, C0 187 and 181.
+// so do the mixed kernels for any scheme and those of ten surfaces and more,
+// where the two registers it keeps are spilled (Surfaces::kKeepsCounter).  With
+// it / without, us: one-shot traces of 4e6 rays C1 483/452, C4 320/306, C0
+// 187/181; plans of 8e6 rays C1 and 8 lens surfaces 791/766 (15 surfaces), 22
+// surfaces of all kinds 393/381, 12 aspheres 1566/1546, 16 2620/2637.
 struct EventCounter {
     int key = -1;
     unsigned n = 0;
